@@ -276,13 +276,15 @@ __global__ void __launch_bounds__(32 * (2 + EW), 1)
       const bool live = m_at < p.m && n_at < p.n;
       // The group's 64 bias values go to shared memory before the accumulator is
       // waited for (their latency hides behind the wait). The four warps of a
-      // group write the same bytes; a slot is reused every third tile, which the
-      // accumulator hand-over below keeps apart from any warp still reading it.
+      // group write the same bytes, whether or not their own rows are live (a
+      // ragged tile's dead warps share the slot with live ones); a slot is reused
+      // every third tile, which the accumulator hand-over below keeps apart from
+      // any warp still reading it.
       uint8_t* bslot = bias_slots + (slot * 4 + group) * 128;
       if (bias != nullptr) {
         const int c = n_at + 2 * lane;
         *reinterpret_cast<uint32_t*>(bslot + 4 * lane) =
-            (live && c < p.n) ? __ldg(reinterpret_cast<const uint32_t*>(bias + c)) : 0u;
+            c < p.n ? __ldg(reinterpret_cast<const uint32_t*>(bias + c)) : 0u;
       }
       if (!mbar_wait(&acc_full[as], aph, p.status)) break;
       tc_fence_after();

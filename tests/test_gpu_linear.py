@@ -221,6 +221,7 @@ def test_qkv_prologue_excludes_the_other_epilogues():
     (4964, 1000, 512, dict(bias=True, act=1, scale=0.5)),  # sixteen epilogue warps (per-warp slabs), ragged rows and columns
     (4900, 1096, 2048, dict(act=1)),                       # sixteen warps without a bias, rows ragged inside a 32-row slab
     (4864, 1024, 512, dict(act=3)),                                        # tanh GELU, four column groups
+    (4930, 1024, 512, dict(bias=True, act=1)),             # a last tile with warps that own no live row
 ])
 def test_cta_pair_gemm_matches_the_oracle(m, n, k, kw):
     """Shapes with at least one 256 x 256 tile per CTA pair run the
