@@ -720,7 +720,16 @@ int attend(const char* OP, const svodb_tensor* q, const svodb_tensor* k, const s
     launch_combine(c, s);
   };
   const bool exact_only = config_lookup("attention|exact") != 0;
-  if (!exact_only && attention_tc_p_covers(a) && config_lookup("attention|one_item") == 0) {
+  const bool one_item = config_lookup("attention|one_item") != 0;
+  if (!exact_only && !one_item && attention_decode_covers(a)) {
+    int rc = launch_attention_decode(a, s, cfg, sizeof cfg);
+    if (rc < 0) return fail(SVODB_ERR_LAUNCH, "%s: the tensor map or kernel attributes were rejected", OP);
+    if (rc == 0) {
+      chose_kernel(OP, packed ? "flash_attention_packed" : "flash_attention", cfg);
+      return check_launch(OP);
+    }
+  }
+  if (!exact_only && !one_item && attention_tc_p_covers(a)) {
     int rc = launch_attention_tc_p(a, s, cfg, sizeof cfg);
     if (rc < 0) return fail(SVODB_ERR_LAUNCH, "%s: the tensor map or kernel attributes were rejected", OP);
     if (rc == 0) {

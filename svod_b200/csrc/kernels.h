@@ -156,6 +156,11 @@ bool attention_tc_covers(const AttnArgs& a);
 int launch_attention_tc_p(const AttnArgs& a, cudaStream_t s, char* cfg, size_t cfg_len);
 bool attention_tc_p_covers(const AttnArgs& a);
 
+// Few query rows per KV head against many keys (cache slices, row maps, appended
+// rows, bool masks, bias): the keys are read once for all of them; same contract.
+int launch_attention_decode(const AttnArgs& a, cudaStream_t s, char* cfg, size_t cfg_len);
+bool attention_decode_covers(const AttnArgs& a);
+
 // The split count an attention over `keys` keys (cached + appended) really runs
 // with: a request is capped at the number of 32-key tiles, so no split is empty
 // by construction.

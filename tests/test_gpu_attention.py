@@ -620,3 +620,60 @@ def test_f16_scores_stay_in_f32_on_the_tensor_core_kernel():
     got = host(ops.attention(dev(q, dt), dev(k, dt), dev(v, dt)))
     assert "kernel flash_attention" in ops.chosen()
     assert np.isfinite(got).all() and np.abs(got - 1.0).max() < 1e-3
+
+
+# Few query rows on many keys: blocks of 128 keys, chunks of 16 query rows, clusters of 1..16 shares.
+DECODE_CASES = [
+    # B, T, Tk, H, Hkv, D, appended, mask
+    (1, 1, 127, 1, 1, 64, 0, "lens"),        # one partial block, one share
+    (2, 1, 128, 4, 4, 128, 0, None),         # exactly one block
+    (3, 4, 129, 8, 2, 64, 1, "lens"),        # all 16 rows of a chunk; a one-key block; one appended row
+    (1, 1, 4100, 2, 1, 128, 0, "lens"),      # sixteen shares of one lane, the last ones short
+    (2, 5, 700, 8, 2, 48, 7, "lens"),        # 20 rows: two chunks, zero-filled head columns
+    (2, 8, 300, 16, 2, 128, 130, "lens"),    # 64 rows, appended rows in two blocks
+    (200, 1, 60, 4, 4, 64, 3, "lens"),       # more (lane, head) pairs than the chip holds
+    (2, 3, 513, 4, 4, 128, 0, "bool"),       # a bool mask with holes
+]
+
+
+@pytest.mark.parametrize("B,T,Tk,H,Hkv,D,appended,mask", DECODE_CASES)
+def test_few_query_rows_on_many_keys(B, T, Tk, H, Hkv, D, appended, mask):
+    """The keys past a lane's length are NaN: they must not reach the result. The weights
+    go through the product as value + remainder, so the result is the f64 oracle's up to
+    the output's rounding: one step of bf16 below magnitude 2, 2^-7."""
+    dt = O.BF16
+    rng = np.random.default_rng(B * 1000 + Tk)
+    q = normal(rng, (B, T, H, D), 1.0, dt)
+    k, v = normal(rng, (B, Tk, Hkv, D), 1.0, dt), normal(rng, (B, Tk, Hkv, D), 0.25, dt)
+    ka, va = normal(rng, (B, appended, Hkv, D), 1.0, dt), normal(rng, (B, appended, Hkv, D), 0.25, dt)
+    lens = rng.integers(0, Tk + 1, B)
+    lens[0] = Tk if B == 1 else 0
+    km = rng.random((B, Tk)) < 0.7
+    kw = dict(key_lens=lens) if mask == "lens" else dict(key_mask=km) if mask == "bool" else {}
+    a = ops.Attn(want_lse=not appended)
+    if mask == "lens":
+        a.keys = ops.KeyMask.Lens(torch.tensor(lens, dtype=torch.int32).cuda())
+    elif mask == "bool":
+        a.keys = ops.KeyMask.Bool(torch.from_numpy(km).cuda())
+    if appended:
+        kw["cache"] = dict(head_start=0, kv_heads=Hkv, row_map=None, k_app=ka, v_app=va, app_lens=None)
+        a.cache = ops.Cache(0, Hkv, None, (dev(ka, dt), dev(va, dt)))
+    want = O.attention(q, k, v, dtype=dt, **kw)
+    K, V = dev(k, dt), dev(v, dt)
+    if mask == "lens":
+        past = (torch.arange(Tk)[None, :] >= torch.from_numpy(lens)[:, None]).cuda()
+        K[past] = float("nan")
+        V[past] = float("nan")
+    out = ops.attention(dev(q, dt), K, V, a)
+    assert "cluster:" in ops.chosen(), ops.chosen()
+    ops.device_status()
+    got = host(out[0] if a.want_lse else out)
+    assert np.isfinite(got).all() and max_abs(got, want) <= 2.0 ** -7
+    if a.want_lse:
+        s = np.einsum("bthd,bjhd->bhtj", q, np.repeat(k, H // Hkv, 2)) / math.sqrt(D)
+        hide = ~km if mask == "bool" else np.arange(Tk)[None, :] >= (lens if mask == "lens" else np.full(B, Tk))[:, None]
+        s = np.where(hide[:, None, None, :], -np.inf, s)
+        with np.errstate(divide="ignore", invalid="ignore"):
+            ref = np.log(np.exp(s - s.max(-1, keepdims=True)).sum(-1)) + s.max(-1)
+        seen = ~np.isnan(ref)
+        assert np.abs(host(out[1])[seen] - ref[seen]).max() < 1e-3 and np.all(np.isneginf(host(out[1])[~seen]))
