@@ -158,6 +158,11 @@ typedef struct svodb_linear_opts {
 /* Bytes of `workspace` a split-K linear of m rows, n columns needs (0 for k_splits <= 1). */
 size_t svodb_linear_workspace_bytes(int64_t m, int64_t n, int32_t k_splits);
 
+/* Or'ed into `svodb_linear_opts.act`: no launch that may still be in flight on the stream
+ * writes `w` (a model's weights). Its first tiles may then be read before the previous
+ * kernel of the stream has finished. */
+#define SVODB_LINEAR_W_STATIC 0x100
+
 /* `ops::linear(x, w, opts)` (tk/src/ops/linear.rs:63-191):
  * y[lead..., N] = scale*act(x[lead..., K] . w[N,K]^T + bias) + residual. */
 int svodb_linear(const svodb_tensor* x, const svodb_tensor* w, const svodb_linear_opts* opts, svodb_tensor* y,

@@ -13,6 +13,7 @@ import os
 # SVODB_LIB_PATH selects another build of the library (e.g. one with debug probes).
 LIB_PATH = Path(os.environ.get("SVODB_LIB_PATH") or Path(__file__).resolve().parent / "lib" / "libsvodb.so")
 
+LINEAR_W_STATIC = 0x100
 MAX_RANK = 5
 
 # status codes of include/svodb.h

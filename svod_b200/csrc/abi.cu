@@ -323,6 +323,7 @@ int svodb_linear(const svodb_tensor* x, const svodb_tensor* w, const svodb_linea
   GUARD(OP);
   svodb_linear_opts none{};
   if (opts == nullptr) opts = &none;
+  const int act = opts->act & ~SVODB_LINEAR_W_STATIC;
   TRY(realized(OP, "x", x));
   TRY(realized(OP, "w", w));
   TRY(realized(OP, "y", y));
@@ -358,7 +359,7 @@ int svodb_linear(const svodb_tensor* x, const svodb_tensor* w, const svodb_linea
   int qkv_per_batch = 0;
   if (qo != nullptr) {
     // The `ops::heads` prologue in the store: same checks as `svodb_heads`.
-    if (rope || opts->gated || opts->act != SVODB_ACT_NONE || opts->has_scale || opts->residual != nullptr)
+    if (rope || opts->gated || act != SVODB_ACT_NONE || opts->has_scale || opts->residual != nullptr)
       return fail(SVODB_ERR_GRAPH, "%s: the qkv prologue excludes rope, gate, activation, scale and residual", OP);
     const int H = qo->heads, Hkv = qo->kv_heads, d = qo->head_dim;
     if (!(Hkv > 0 && H > 0 && H % Hkv == 0))
@@ -423,12 +424,13 @@ int svodb_linear(const svodb_tensor* x, const svodb_tensor* w, const svodb_linea
   a.ldw = k;
   a.ldc = y->rank >= 2 ? y->stride[y->rank - 2] : n;
   a.ldr = opts->residual ? (opts->residual->rank >= 2 ? opts->residual->stride[opts->residual->rank - 2] : n) : 0;
-  a.act = opts->act;
+  a.act = act;
   a.gated = opts->gated;
   a.has_scale = opts->has_scale;
   a.scale = opts->scale;
   a.dtype = x->dtype;
   a.status = device_status_word();
+  a.w_static = (opts->act & SVODB_LINEAR_W_STATIC) != 0;
   if (a.m == 0 || n == 0) {
     chose_graph(OP, "shape");
     return SVODB_OK;
@@ -453,7 +455,7 @@ int svodb_linear(const svodb_tensor* x, const svodb_tensor* w, const svodb_linea
     const char* epi = qo != nullptr ? "qkv" : rope ? "rope" : opts->gated ? "gated" : "plain";
     char key[160];
     snprintf(key, sizeof key, "gemm|%s|%lld|%lld|%lld|%s%s%s", dtype_name(x->dtype), (long long)a.m, (long long)n,
-             (long long)k, epi, opts->residual != nullptr ? "+res" : "", opts->act != SVODB_ACT_NONE ? "+act" : "");
+             (long long)k, epi, opts->residual != nullptr ? "+res" : "", act != SVODB_ACT_NONE ? "+act" : "");
     a.force_bn = config_lookup(key);
     if (gemm_tc_covers(a)) snprintf(g_config_key, sizeof g_config_key, "%s", key);
   }
@@ -474,6 +476,15 @@ int svodb_linear(const svodb_tensor* x, const svodb_tensor* w, const svodb_linea
     f.norm_k_heads = qo->kv_heads;
     f.norm_eps = (float)qo->eps;
     const bool any = f.rope_cos != nullptr || f.norm_q != nullptr || f.norm_k != nullptr;
+    if (any && (f.force_bn == 0 || f.force_bn >= kForceSmall)) {
+      const int splits = gemm_small_splits(f);
+      if (splits > 0) {
+        if (launch_gemm_small(f, splits, s, cfg, sizeof cfg) != 0)
+          return fail(SVODB_ERR_LAUNCH, "%s: the tensor map or kernel attributes were rejected", OP);
+        chose_kernel(OP, "gemm", cfg);
+        return check_launch(OP);
+      }
+    }
     if (any && (f.force_bn == 512 ? gemm_tc2_covers(f) : (f.force_bn == 0 && gemm_tc2_preferred(f)))) {
       int rc = launch_gemm_tc2(f, s, cfg, sizeof cfg);
       if (rc < 0) return fail(SVODB_ERR_LAUNCH, "%s: the tensor map or kernel attributes were rejected", OP);
@@ -510,6 +521,16 @@ int svodb_linear(const svodb_tensor* x, const svodb_tensor* w, const svodb_linea
         chose_kernel(OP, "gemm", cfg);
         return check_launch(OP);
       }
+    }
+  }
+  if (a.force_bn == 0 || a.force_bn >= kForceSmall) {
+    const int splits = gemm_small_splits(a);
+    if (splits > 0) {
+      if (launch_gemm_small(a, splits, s, cfg, sizeof cfg) != 0)
+        return fail(SVODB_ERR_LAUNCH, "%s: the tensor map or kernel attributes were rejected", OP);
+      chose_kernel(OP, "gemm", cfg);
+      if (qo != nullptr) heads_in_place(qo, y, qkv_per_batch, s);
+      return check_launch(OP);
     }
   }
   if (a.force_bn == 512 ? gemm_tc2_covers(a) : (a.force_bn == 0 && gemm_tc2_preferred(a))) {

@@ -45,6 +45,7 @@
 #include "attention_parts.cuh"
 #include "common.cuh"
 #include "kernels.h"
+#include "launch.h"
 #include "svodb.h"
 #include "tensormap.h"
 
@@ -191,6 +192,7 @@ __global__ void __launch_bounds__(kThreadsDec, (DecCfg<D, NQ>::kPerSm))
   const int pair = blockIdx.x / csize;
   const int b = pair / p.kv_heads, hk = pair % p.kv_heads;
 
+  pdl_wait();
   // This lane's visible keys and this CTA's share of their blocks.
   int64_t kv_row = p.row_map != nullptr ? (int64_t)p.row_map[b] : b;
   const bool bad_row = kv_row < 0 || kv_row >= p.kv_rows;
@@ -270,6 +272,7 @@ __global__ void __launch_bounds__(kThreadsDec, (DecCfg<D, NQ>::kPerSm))
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
+  pdl_trigger();
   const uint32_t tmem_base = *tmem_slot;
 
   if (warp == 4) {
@@ -645,19 +648,9 @@ int run_dec(const AttnArgs& a, cudaStream_t s, char* cfg, size_t cfg_len) {
   while (csize < 16 && csize * 2 <= blocks &&
          (pairs * csize * 2 <= room || (pairs * csize < 4 * room && blocks >= 32 * csize * 2)))
     csize *= 2;
-  cudaLaunchConfig_t lc{};
-  lc.gridDim = dim3((unsigned)(pairs * csize), 1, 1);
-  lc.blockDim = dim3(kThreadsDec, 1, 1);
-  lc.dynamicSmemBytes = C::kSmem;
-  lc.stream = s;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = (unsigned)csize;
-  attr[0].val.clusterDim.y = 1;
-  attr[0].val.clusterDim.z = 1;
-  lc.attrs = attr;
-  lc.numAttrs = 1;
-  if (cudaLaunchKernelEx(&lc, attention_decode_kernel<T, D, NQ>, tk, tv, tka, tva, p) != cudaSuccess) return -1;
+  if (launch_pdl(attention_decode_kernel<T, D, NQ>, dim3((unsigned)(pairs * csize)), dim3(kThreadsDec), C::kSmem, s,
+                 (unsigned)csize, tk, tv, tka, tva, p) != cudaSuccess)
+    return -1;
   if (cfg != nullptr)
     snprintf(cfg, cfg_len, "{rows:%d,bkv:%d,d:%d,stages:%d,splits:1,cluster:%d}", NQ, kKeys, a.d, C::kSlots, csize);
   return 0;

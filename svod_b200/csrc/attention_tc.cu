@@ -50,6 +50,7 @@
 #include "attention_parts.cuh"
 #include "common.cuh"
 #include "kernels.h"
+#include "launch.h"
 #include "svodb.h"
 #include "tensormap.h"
 
@@ -123,6 +124,8 @@ __global__ void __launch_bounds__(kThreadsFa, 1)
     tmem_relinquish();
   }
   __syncthreads();
+  pdl_trigger();
+  pdl_wait();
   // ---- key mask scan (warps 2-3): prefix length, or a bitmask -----------------
   if (p.key_mask != nullptr && (warp == 2 || warp == 3)) {
     const int tid = threadIdx.x - 64;
@@ -641,7 +644,8 @@ int run(const AttnArgs& a, cudaStream_t s, char* cfg, size_t cfg_len) {
   p.d_real = a.d;
   p.status = a.status;
   dim3 grid((unsigned)p.n_qt, (unsigned)a.heads, (unsigned)a.batch);
-  attention_tc_kernel<T, D><<<grid, kThreadsFa, C::kSmemBytes, s>>>(tq, tk, tv, p);
+  if (launch_pdl(attention_tc_kernel<T, D>, grid, dim3(kThreadsFa), C::kSmemBytes, s, 1, tq, tk, tv, p) != cudaSuccess)
+    return -1;
   if (cfg != nullptr)
     snprintf(cfg, cfg_len, "{bq:%d,bkv:%d,d:%d,stages:%d,splits:1}", 2 * kBQ, kBKV, a.d, C::kStages);
   return 0;

@@ -35,6 +35,7 @@
 #include "attention_parts.cuh"
 #include "common.cuh"
 #include "kernels.h"
+#include "launch.h"
 #include "svodb.h"
 #include "tensormap.h"
 
@@ -44,8 +45,9 @@ namespace {
 
 using namespace fa_parts;
 
-// Queue heads: items handed out so far by a running launch, one per (device,
-// stream) pair, zeroed on the stream just before each launch.
+// Queue heads: items handed out so far by a running launch and CTAs that are done with
+// it, one pair per (device, stream). Both are zero between launches: the CTA that is
+// done last puts them back, so that no memset stands between two kernels of a stream.
 constexpr int kQueueSlots = 256;
 // Output staging of the softmax warps: a 32-row x 64-column slab each, stored by TMA.
 constexpr int kOutStageBytes = 8 * 32 * 128;
@@ -54,7 +56,7 @@ constexpr size_t smem_bytes_p() {
   using C = FaCfg<D>;
   return 1024 + (size_t)2 * C::kQTileBytes + (size_t)2 * C::kStages * C::kKvBytes + kOutStageBytes + 512;
 }
-__device__ int g_next_item[kQueueSlots];
+__device__ int g_next_item[2 * kQueueSlots];
 
 struct Item {
   int qt, h, b, valid;
@@ -120,7 +122,7 @@ __device__ __forceinline__ void scan_mask_row(const FaParams& p, int64_t b, int 
     const uint4* row = reinterpret_cast<const uint4*>((const uint8_t*)p.key_mask + base);
     const int pieces = (int)(p.tk >> 4);
     for (int c = lane; c < pieces; c += 32) {
-      const uint4 u = __ldg(row + c);
+      const uint4 u = ldg128(row + c);
       const uint32_t wd[4] = {u.x, u.y, u.z, u.w};
 #pragma unroll
       for (int q = 0; q < 4; ++q) {
@@ -267,6 +269,8 @@ __global__ void __launch_bounds__(kThreadsFa, 1)
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
+  pdl_trigger();
+  pdl_wait();
   const uint32_t tmem_base = *tmem_slot;
 
   auto plan = [&](const Item& it, const MaskRow& mrow) -> Work {
@@ -808,6 +812,11 @@ __global__ void __launch_bounds__(kThreadsFa, 1)
 
   tc_fence_before();
   __syncthreads();
+  if (threadIdx.x == 0 && atomicAdd(queue + 1, 1) == (int)gridDim.x - 1) {
+    // every CTA has taken its last item: the queue is as the next launch wants it
+    queue[0] = 0;
+    queue[1] = 0;
+  }
   if (warp == 2) {
     __syncwarp();
     tc_fence_after();
@@ -841,7 +850,7 @@ int* queue_head(cudaStream_t stream) {
     if (used >= kQueueSlots) return nullptr;
     it = slots.emplace(key, used).first;
   }
-  return base[dev] + it->second;
+  return base[dev] + 2 * it->second;
 }
 
 // An item is one 128-row tile of two query heads (instead of two tiles of one head)
@@ -938,9 +947,9 @@ int run_p(const AttnArgs& a, cudaStream_t s, char* cfg, size_t cfg_len) {
     const int64_t want = (6 * (int64_t)sms + per_kv - 1) / per_kv;
     tail_groups = (int)(want < groups ? want : groups);
   }
-  if (cudaMemsetAsync(head, 0, sizeof(int), s) != cudaSuccess) return -1;
-  attention_tc_p_kernel<T, D, EXTRAS><<<grid, kThreadsFa, smem_bytes_p<D>(), s>>>(tq, tk, tv, to, p, (int)items,
-                                                                                  tail_groups, head);
+  if (launch_pdl(attention_tc_p_kernel<T, D, EXTRAS>, dim3((unsigned)grid), dim3(kThreadsFa), smem_bytes_p<D>(), s, 1, tq, tk,
+                 tv, to, p, (int)items, tail_groups, head) != cudaSuccess)
+    return -1;
   if (cfg != nullptr)
     snprintf(cfg, cfg_len, p.pair_heads ? "{bq:%d,bkv:%d,d:%d,stages:%d,splits:%d,persistent:%d,head_pairs:1}"
                                         : "{bq:%d,bkv:%d,d:%d,stages:%d,splits:%d,persistent:%d}",

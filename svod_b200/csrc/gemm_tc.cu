@@ -28,6 +28,7 @@
 #include "common.cuh"
 #include "gemm_parts.cuh"
 #include "kernels.h"
+#include "launch.h"
 #include "svodb.h"
 #include "tensormap.h"
 
@@ -152,6 +153,7 @@ __global__ void __launch_bounds__(kThreads, 1)
     tmem_alloc(tmem_slot, C::kTmemCols);
     tmem_relinquish();
   }
+  pdl_wait();
   if ((p.head_epilogue || p.head64_epilogue) && threadIdx.x < 256) {
     const T* wsrc = (const T*)(threadIdx.x < 128 ? p.norm_q : p.norm_k);
     const int at = threadIdx.x & 127;
@@ -160,6 +162,7 @@ __global__ void __launch_bounds__(kThreads, 1)
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
+  pdl_trigger();
   const uint32_t tmem_base = *tmem_slot;
 
   if (warp == 0) {
@@ -686,7 +689,9 @@ int run(const GemmArgs& a, const Params& p0, int sms, cudaStream_t s, char* cfg,
   }
   const int tiles = p.tiles_m * p.tiles_n;
   const int grid = tiles < sms ? tiles : sms;
-  gemm_tc_kernel<T, BN><<<grid, kThreads, C::kSmemBytes, s>>>(ta, tw, tc, tr, p);
+  if (launch_pdl(gemm_tc_kernel<T, BN>, dim3((unsigned)grid), dim3(kThreads), C::kSmemBytes, s, 1, ta, tw, tc, tr, p) !=
+      cudaSuccess)
+    return -1;
   if (cfg != nullptr)
     snprintf(cfg, cfg_len, "{bm:%d,bn:%d,bk:%d,stages:%d,gated:%d,grid:%d}", BM, BN, BK, C::kStages, a.gated, grid);
   return 0;

@@ -24,6 +24,7 @@
 #include "common.cuh"
 #include "gemm_parts.cuh"
 #include "kernels.h"
+#include "launch.h"
 #include "svodb.h"
 #include "tensormap.h"
 
@@ -135,6 +136,7 @@ __global__ void __launch_bounds__(32 * (2 + EW), 1)
     tmem_alloc_pair(tmem_slot, kTmemCols);
     tmem_relinquish_pair();
   }
+  pdl_wait();
   if (HEADS && threadIdx.x < 256) {
     const T* wsrc = (const T*)(threadIdx.x < 128 ? p.norm_q : p.norm_k);
     head_w[threadIdx.x] = wsrc != nullptr ? Elem<T>::to_f(wsrc[threadIdx.x & 127]) : 1.0f;
@@ -144,6 +146,7 @@ __global__ void __launch_bounds__(32 * (2 + EW), 1)
   // The partner's barriers must exist before anything signals them.
   cluster_sync_all();
   tc_fence_after();
+  pdl_trigger();
   const uint32_t tmem_base = *tmem_slot;
 
   if (warp == 0) {
@@ -284,7 +287,7 @@ __global__ void __launch_bounds__(32 * (2 + EW), 1)
       if (bias != nullptr) {
         const int c = n_at + 2 * lane;
         *reinterpret_cast<uint32_t*>(bslot + 4 * lane) =
-            c < p.n ? __ldg(reinterpret_cast<const uint32_t*>(bias + c)) : 0u;
+            c < p.n ? *reinterpret_cast<const volatile uint32_t*>(bias + c) : 0u;
       }
       if (!mbar_wait(&acc_full[as], aph, p.status)) break;
       tc_fence_after();
@@ -704,19 +707,9 @@ int run2(const GemmArgs& a, int sms, cudaStream_t s, char* cfg, size_t cfg_len) 
   }
   const int tiles = p.tiles_m * p.tiles_n;
   const int pairs = tiles < sms / 2 ? tiles : sms / 2;
-  cudaLaunchConfig_t lc{};
-  lc.gridDim = dim3((unsigned)(2 * pairs), 1, 1);
-  lc.blockDim = dim3(C::kThreads, 1, 1);
-  lc.dynamicSmemBytes = C::kSmemBytes;
-  lc.stream = s;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = 2;
-  attr[0].val.clusterDim.y = 1;
-  attr[0].val.clusterDim.z = 1;
-  lc.attrs = attr;
-  lc.numAttrs = 1;
-  if (cudaLaunchKernelEx(&lc, gemm_tc2_kernel<T, HEADS, EW>, ta, tw, tc, tr, tcos, tsin, p) != cudaSuccess) return -1;
+  if (launch_pdl(gemm_tc2_kernel<T, HEADS, EW>, dim3((unsigned)(2 * pairs)), dim3(C::kThreads), C::kSmemBytes, s, 2, ta, tw,
+                 tc, tr, tcos, tsin, p) != cudaSuccess)
+    return -1;
   if (cfg != nullptr)
     snprintf(cfg, cfg_len, "{bm:%d,bn:%d,bk:%d,stages:%d,gated:%d,grid:%d,cta_pair:1,epi_warps:%d}", 2 * BM, BN, BK,
              C::kStages, a.gated, 2 * pairs, EW);

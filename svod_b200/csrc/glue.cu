@@ -3,6 +3,7 @@
 // RoPE tables. All HBM-bound or negligible; written for coalesced access.
 #include "common.cuh"
 #include "kernels.h"
+#include "launch.h"
 #include "rows_parts.cuh"
 #include "svodb.h"
 
@@ -29,6 +30,10 @@ __global__ void __launch_bounds__(256)
   const int64_t t0 = (int64_t)blockIdx.x * kTok;
   const I* row = ids + b * t_len;
   const int tid = threadIdx.x;
+  // The first kernel of a stack: it lets the next one up only once all before it is done,
+  // so that nothing later ever runs beside what was on the stream before the stack.
+  pdl_wait();
+  pdl_trigger();
   int before = 0;
   if (pos_table != nullptr && pad_id >= 0) {
     int cnt = 0;
@@ -119,6 +124,8 @@ __global__ void __launch_bounds__(kTok * 32)
   const int64_t t0 = (int64_t)blockIdx.x * kTok;
   const I* row = ids + bi * t_len;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  pdl_wait();  // then the trigger: as in embed_kernel
+  pdl_trigger();
   int before = 0;
   if (pos_table != nullptr && pad_id >= 0) {
     int cnt = 0;
@@ -195,6 +202,8 @@ __global__ void __launch_bounds__(256)
   __shared__ float part[8192];  // [warps][D], warps * D <= 8192
   __shared__ float cnts[8];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
+  pdl_trigger();
+  pdl_wait();
   const int64_t bi = mode == 3 ? blockIdx.x / slots : blockIdx.x;
   const T* h = hidden + bi * l_len * D;
   float acc[SPANS][8];
@@ -392,9 +401,8 @@ void launch_embed(const EmbedArgs& a, cudaStream_t s) {
   dim3 grid((unsigned)((a.t + kTok - 1) / kTok), (unsigned)a.batch);
   const int vec16 = aligned16(a.table) && aligned16(a.pos_table) && aligned16(a.type_row) && aligned16(a.out) ? 1 : 0;
 #define SVODB_EMBED(T, I)                                                                                         \
-  embed_kernel<T, I><<<grid, 256, 0, s>>>((const I*)a.ids, (const T*)a.table, (const T*)a.pos_table,              \
-                                          (const T*)a.type_row, a.pad_id, (T*)a.out, a.t, a.d, a.vocab, a.max_pos, \
-                                          vec16)
+  launch_pdl(embed_kernel<T, I>, grid, dim3(256), 0, s, 1, (const I*)a.ids, (const T*)a.table,         \
+             (const T*)a.pos_table, (const T*)a.type_row, a.pad_id, (T*)a.out, a.t, a.d, a.vocab, a.max_pos, vec16)
   if (a.dtype == SVODB_BF16) {
     if (a.ids_i64) SVODB_EMBED(__nv_bfloat16, int64_t);
     else SVODB_EMBED(__nv_bfloat16, int32_t);
@@ -411,10 +419,9 @@ bool embed_norm_dispatch(const EmbedArgs& a, const EmbedNormArgs& n, cudaStream_
   dim3 grid((unsigned)((a.t + kTok - 1) / kTok), (unsigned)a.batch);
 #define SVODB_EN(SP)                                                                                                \
   case SP:                                                                                                          \
-    embed_norm_kernel<T, I, SP><<<grid, kTok * 32, 0, s>>>((const I*)a.ids, (const T*)a.table, (const T*)a.pos_table, \
-                                                           (const T*)a.type_row, a.pad_id, (const T*)n.w,             \
-                                                           (const T*)n.b, n.eps, n.layer, (T*)a.out, a.t, a.vocab,   \
-                                                           a.max_pos);                                               \
+    launch_pdl(embed_norm_kernel<T, I, SP>, grid, dim3(kTok * 32), 0, s, 1, (const I*)a.ids, (const T*)a.table,      \
+               (const T*)a.pos_table, (const T*)a.type_row, a.pad_id, (const T*)n.w, (const T*)n.b, n.eps, n.layer, \
+               (T*)a.out, a.t, a.vocab, a.max_pos);                                                                \
     return true
   switch (a.d / 256) {
     SVODB_EN(1); SVODB_EN(2); SVODB_EN(3); SVODB_EN(4); SVODB_EN(5); SVODB_EN(6); SVODB_EN(7); SVODB_EN(8);
@@ -433,10 +440,9 @@ bool norm_pool_dispatch(const PoolArgs& a, const EmbedNormArgs& n, cudaStream_t 
   const PeerPush pp = a.push != nullptr ? *a.push : PeerPush{};
 #define SVODB_NP(SP)                                                                                               \
   case SP:                                                                                                         \
-    norm_pool_kernel<T, SP><<<(unsigned)out_rows, warps * 32, 0, s>>>((const T*)a.hidden, (const T*)n.w,           \
-                                                                      (const T*)n.b, n.eps, n.layer, a.aux,         \
-                                                                      a.aux_i32, a.mode, a.slots, a.normalize,      \
-                                                                      a.out, a.out_row_stride, a.l, pp);            \
+    launch_pdl(norm_pool_kernel<T, SP>, dim3((unsigned)out_rows), dim3(warps * 32), 0, s, 1, (const T*)a.hidden,    \
+               (const T*)n.w, (const T*)n.b, n.eps, n.layer, a.aux, a.aux_i32, a.mode, a.slots, a.normalize, a.out, \
+               a.out_row_stride, a.l, pp);                                                                         \
     return true
   switch (spans) {
     SVODB_NP(1); SVODB_NP(2); SVODB_NP(3); SVODB_NP(4); SVODB_NP(5); SVODB_NP(6); SVODB_NP(7); SVODB_NP(8);

@@ -11,6 +11,7 @@
 // head's first half and the 8 partner elements of its second half.
 #include "common.cuh"
 #include "kernels.h"
+#include "launch.h"
 #include "svodb.h"
 
 namespace svodb {
@@ -42,6 +43,8 @@ __global__ void __launch_bounds__(256)
                  int per_batch_tables, int in_place) {
   constexpr int D = LPH * 16;
   constexpr int HALF = D / 2;
+  pdl_trigger();
+  pdl_wait();
   const int slots = heads + 2 * kv_heads;
   const int64_t total = tokens * slots;
   const int64_t gthread = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -154,9 +157,9 @@ void run(const HeadsArgs& a, cudaStream_t s) {
   const int64_t tokens = a.batch * a.t;
   const int64_t threads = tokens * (a.heads + 2 * a.kv_heads) * LPH;
   const unsigned blocks = (unsigned)((threads + 255) / 256);
-  heads_kernel<T, LPH><<<blocks, 256, 0, s>>>((const T*)a.qkv, (const T*)a.q_w, (const T*)a.k_w, (const T*)a.cos,
-                                              (const T*)a.sin, (T*)a.q, (T*)a.k, (T*)a.v, tokens, a.t, a.heads,
-                                              a.kv_heads, a.eps, a.per_batch_tables, a.in_place);
+  launch_pdl(heads_kernel<T, LPH>, dim3(blocks), dim3(256), 0, s, 1, (const T*)a.qkv, (const T*)a.q_w, (const T*)a.k_w,
+             (const T*)a.cos, (const T*)a.sin, (T*)a.q, (T*)a.k, (T*)a.v, tokens, a.t, a.heads, a.kv_heads, a.eps,
+             a.per_batch_tables, a.in_place);
 }
 
 template <typename T>

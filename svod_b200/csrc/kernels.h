@@ -215,7 +215,13 @@ struct GemmArgs {
   int k_splits;
   void* workspace;
   size_t workspace_bytes;
+  int w_static;  // the caller's word that no launch in flight writes w: its loads need not wait for one
 };
+// `force_bn` codes of the few-tile kernel: kForceSmall + S = a cluster of S CTAs a tile.
+constexpr int kForceSmall = 1024;
+// The few-tile kernel: CTAs per tile it would run the call with, 0 where another kernel is the better one.
+int gemm_small_splits(const GemmArgs& a);
+int launch_gemm_small(const GemmArgs& a, int splits, cudaStream_t s, char* cfg, size_t cfg_len);
 // Workspace bytes of a split-K GEMM: [tiles][2] counters, then [tiles][splits][2][128][256] f32.
 size_t gemm_splitk_workspace_bytes(int64_t m, int64_t n, int k_splits);
 // Whether the split-K instantiation takes the call (plain epilogue: bias, activation,

@@ -56,6 +56,9 @@ struct svodb_plan {
   cudaStream_t stream;
 };
 
+// Every projection's weights are the model's: no launch in flight writes them
+// (SVODB_LINEAR_W_STATIC); each stack begins with an embedding lookup, which lets nothing
+// up before all that was on the stream is done.
 namespace {
 
 size_t esize_of(int dtype) { return dtype == SVODB_F32 ? 4 : 2; }
@@ -185,27 +188,29 @@ int forward_qwen3(const svodb_plan* p, const Acts& a, int reference_ops) {
     RUN(svodb_rms_norm(&x, &in_w, c.eps, &xn, s));
     if (!reference_ops) {
       svodb_linear_opts lo{};
-      lo.qkv = &pro;
+      lo.qkv = &pro; lo.act |= SVODB_LINEAR_W_STATIC;
       RUN(svodb_linear(&xn, &qkv_w, &lo, &qkv, s));
       RUN(svodb_attention_packed(&qkv, (int32_t)H, (int32_t)Hkv, &causal, &attn4, s));
     } else {
       svodb_tensor q = tensor(a.q, dt, {B, L, H, hd});
       svodb_tensor k = tensor(a.k, dt, {B, L, Hkv, hd});
       svodb_tensor v = tensor(a.v, dt, {B, L, Hkv, hd});
-      RUN(svodb_linear(&xn, &qkv_w, nullptr, &qkv, s));
+      svodb_linear_opts lo{};
+      lo.act = SVODB_LINEAR_W_STATIC;
+      RUN(svodb_linear(&xn, &qkv_w, &lo, &qkv, s));
       RUN(svodb_heads(&qkv, &pro, &q, &k, &v, s));
       RUN(svodb_attention(&q, &k, &v, &causal, &attn4, s));
     }
     svodb_linear_opts oo{};
-    oo.residual = &x;
+    oo.residual = &x; oo.act |= SVODB_LINEAR_W_STATIC;
     RUN(svodb_linear(&attn3, &o_w, &oo, &h, s));
     RUN(svodb_rms_norm(&h, &post_w, c.eps, &hn, s));
     svodb_linear_opts go{};
-    go.act = SVODB_ACT_SILU;
+    go.act = SVODB_ACT_SILU | SVODB_LINEAR_W_STATIC;
     go.gated = 1;
     RUN(svodb_linear(&hn, &gu_w, &go, &g, s));
     svodb_linear_opts dn{};
-    dn.residual = &h;
+    dn.residual = &h; dn.act |= SVODB_LINEAR_W_STATIC;
     RUN(svodb_linear(&g, &down_w, &dn, &x, s));
   }
   // final RMSNorm of the pooled (last real) tokens, pooling, L2: one kernel
@@ -247,18 +252,18 @@ int forward_xlmr(const svodb_plan* p, const Acts& a) {
     svodb_tensor fo_w = tensor(lw.fo_w, dt, {D, F}), fo_b = tensor(lw.fo_b, dt, {D});
     svodb_tensor ln2_w = tensor(lw.ln2_w, dt, {D}), ln2_b = tensor(lw.ln2_b, dt, {D});
     svodb_linear_opts po{};
-    po.bias = &qkv_b;
+    po.bias = &qkv_b; po.act |= SVODB_LINEAR_W_STATIC;
     RUN(svodb_linear(&x, &qkv_w, &po, &qkv, s));
     RUN(svodb_attention_packed(&qkv, (int32_t)H, (int32_t)H, &keys, &attn4, s));
     svodb_linear_opts oo{};
-    oo.bias = &o_b, oo.residual = &x;
+    oo.bias = &o_b, oo.residual = &x; oo.act |= SVODB_LINEAR_W_STATIC;
     RUN(svodb_linear(&attn3, &o_w, &oo, &y, s));
     RUN(svodb_layer_norm(&y, &ln1_w, &ln1_b, c.eps, &x1, s));
     svodb_linear_opts fi{};
-    fi.bias = &fi_b, fi.act = SVODB_ACT_GELU;
+    fi.bias = &fi_b, fi.act = SVODB_ACT_GELU | SVODB_LINEAR_W_STATIC;
     RUN(svodb_linear(&x1, &fi_w, &fi, &f, s));
     svodb_linear_opts fo{};
-    fo.bias = &fo_b, fo.residual = &x1;
+    fo.bias = &fo_b, fo.residual = &x1; fo.act |= SVODB_LINEAR_W_STATIC;
     RUN(svodb_linear(&f, &fo_w, &fo, &y, s));
     RUN(svodb_layer_norm(&y, &ln2_w, &ln2_b, c.eps, &x, s));
   }
@@ -310,7 +315,7 @@ int forward_modernbert(const svodb_plan* p, const Acts& a) {
     po.rope_cos = global ? &cos_g : &cos_l;
     po.rope_sin = global ? &sin_g : &sin_l;
     po.rope_heads = (int32_t)(2 * H);
-    po.rope_head_dim = (int32_t)hd;
+    po.rope_head_dim = (int32_t)hd; po.act |= SVODB_LINEAR_W_STATIC;
     RUN(svodb_linear(src, &qkv_w, &po, &qkv, s));
     svodb_attn_opts ao{};
     ao.key_mask = &mask;
@@ -320,15 +325,15 @@ int forward_modernbert(const svodb_plan* p, const Acts& a) {
     }
     RUN(svodb_attention_packed(&qkv, (int32_t)H, (int32_t)H, &ao, &attn4, s));
     svodb_linear_opts oo{};
-    oo.residual = &x;
+    oo.residual = &x; oo.act |= SVODB_LINEAR_W_STATIC;
     RUN(svodb_linear(&attn3, &o_w, &oo, &h, s));
     RUN(svodb_layer_norm(&h, &mlp_w, nullptr, c.eps, &hn, s));
     svodb_linear_opts go{};
-    go.act = SVODB_ACT_GELU;
+    go.act = SVODB_ACT_GELU | SVODB_LINEAR_W_STATIC;
     go.gated = 1;
     RUN(svodb_linear(&hn, &wi_w, &go, &g, s));
     svodb_linear_opts dn{};
-    dn.residual = &h;
+    dn.residual = &h; dn.act |= SVODB_LINEAR_W_STATIC;
     RUN(svodb_linear(&g, &wo_w, &dn, &x, s));
   }
   // final LayerNorm of the pooled tokens, pooling, L2: one kernel

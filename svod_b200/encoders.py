@@ -110,21 +110,23 @@ class XlmRobertaEncoder:
         # lookup (word + position + type) and the embedding LayerNorm: one kernel
         x = ops.embed_norm(ids, p["word"], p["emb_ln_w"], p["emb_ln_b"], c.layer_norm_eps, p["pos"], p["type"],
                            c.pad_token_id)
-        return self.run_layers(x, mask)
+        return self.run_layers(x, mask, w_static=True)
 
-    def run_layers(self, x: torch.Tensor, mask: torch.Tensor, start: int = 0, stop: Optional[int] = None):
-        """Layers `start .. stop` over the hidden states `x [B,L,D]`."""
+    def run_layers(self, x: torch.Tensor, mask: torch.Tensor, start: int = 0, stop: Optional[int] = None,
+                   w_static: bool = False):
+        """Layers `start .. stop` over the hidden states `x [B,L,D]`. `w_static`: behind the
+        stack's own embedding lookup, no launch in flight writes the weights."""
         c, p = self.cfg, self.p
         H = c.num_attention_heads
         B, L, D = x.shape
         keys = KeyMask.Bool(mask)
         for lp in p["layers"][start:stop]:
-            qkv = ops.linear(x, lp["qkv_w"], Linear(bias=lp["qkv_b"]))
+            qkv = ops.linear(x, lp["qkv_w"], Linear(bias=lp["qkv_b"], w_static=w_static))
             a = ops.attention_packed(qkv, H, H, Attn(keys=keys)).view(B, L, D)
-            y = ops.linear(a, lp["o_w"], Linear(bias=lp["o_b"], residual=x))
+            y = ops.linear(a, lp["o_w"], Linear(bias=lp["o_b"], residual=x, w_static=w_static))
             x = ops.layer_norm(y, lp["ln1_w"], lp["ln1_b"], c.layer_norm_eps)
-            f = ops.linear(x, lp["fi_w"], Linear(bias=lp["fi_b"], act=Act.GELU))
-            y = ops.linear(f, lp["fo_w"], Linear(bias=lp["fo_b"], residual=x))
+            f = ops.linear(x, lp["fi_w"], Linear(bias=lp["fi_b"], act=Act.GELU, w_static=w_static))
+            y = ops.linear(f, lp["fo_w"], Linear(bias=lp["fo_b"], residual=x, w_static=w_static))
             x = ops.layer_norm(y, lp["ln2_w"], lp["ln2_b"], c.layer_norm_eps)
         return x
 
@@ -166,12 +168,14 @@ class Qwen3Embedder:
                rope=None) -> torch.Tensor:
         c, p = self.cfg, self.p
         H, Hkv, hd = c.num_attention_heads, c.num_key_value_heads, c.head_dim
-        x = self.run_layers(ops.embed(ids, p["embed"]), seg_start, rope)
+        x = self.run_layers(ops.embed(ids, p["embed"]), seg_start, rope, w_static=True)
         return ops.rms_norm(x, p["norm_w"], c.rms_norm_eps)
 
     def run_layers(self, x: torch.Tensor, seg_start: Optional[torch.Tensor] = None, rope=None, start: int = 0,
-                   stop: Optional[int] = None) -> torch.Tensor:
-        """Layers `start .. stop` over the hidden states `x [B,L,D]` (no final norm)."""
+                   stop: Optional[int] = None, w_static: bool = False) -> torch.Tensor:
+        """Layers `start .. stop` over the hidden states `x [B,L,D]` (no final norm).
+        `w_static`: behind the stack's own embedding lookup, no launch in flight writes
+        the weights."""
         c, p = self.cfg, self.p
         H, Hkv, hd = c.num_attention_heads, c.num_key_value_heads, c.head_dim
         B, L, D = x.shape
@@ -182,21 +186,21 @@ class Qwen3Embedder:
             if self.fused_prologue:
                 # q/k norm and rotation in the projection's store; attention reads
                 # the packed projection in place (no q, k, v copies).
-                qkv = ops.linear(xn, lp["qkv_w"], Linear(qkv=prologue))
+                qkv = ops.linear(xn, lp["qkv_w"], Linear(qkv=prologue, w_static=w_static))
                 a = ops.attention_packed(qkv, H, Hkv, Attn(causal=True, seg_start=seg_start)).view(B, L, H * hd)
             else:
                 # the reference's op sequence (model/src/qwen3/attention.rs:69-113)
-                q, k, v = ops.heads(ops.linear(xn, lp["qkv_w"]), prologue)
+                q, k, v = ops.heads(ops.linear(xn, lp["qkv_w"], Linear(w_static=w_static)), prologue)
                 a = ops.attention(q, k, v, Attn(causal=True, seg_start=seg_start)).view(B, L, H * hd)
-            h = ops.linear(a, lp["o_w"], Linear(residual=x))
+            h = ops.linear(a, lp["o_w"], Linear(residual=x, w_static=w_static))
             hn = ops.rms_norm(h, lp["post_w"], c.rms_norm_eps)
-            g = ops.linear(hn, lp["gu_w"], Linear(act=Act.SILU, gated=True))
-            x = ops.linear(g, lp["down_w"], Linear(residual=h))
+            g = ops.linear(hn, lp["gu_w"], Linear(act=Act.SILU, gated=True, w_static=w_static))
+            x = ops.linear(g, lp["down_w"], Linear(residual=h, w_static=w_static))
         return x
 
     def forward(self, ids, lengths, out=None, gather=None):
         # final RMSNorm of the pooled (last real) tokens alone, pooling and L2: one kernel
-        x = self.run_layers(ops.embed(ids, self.p["embed"]))
+        x = self.run_layers(ops.embed(ids, self.p["embed"]), w_static=True)
         return ops.norm_pool(x, self.p["norm_w"], None, self.cfg.rms_norm_eps, layer=False, aux=lengths,
                              mode=ops.POOL_LAST, out=out, gather=gather)
 
@@ -235,10 +239,13 @@ class ModernBertEncoder:
         H = c.num_attention_heads
         hd = c.hidden_size // H
         x = ops.embed_norm(ids, p["embed"], p["emb_ln_w"], None, c.norm_eps)
-        return ops.layer_norm(self.run_layers(x, mask), p["final_ln_w"], None, c.norm_eps)
+        return ops.layer_norm(self.run_layers(x, mask, w_static=True), p["final_ln_w"], None, c.norm_eps)
 
-    def run_layers(self, x: torch.Tensor, mask: torch.Tensor, start: int = 0, stop: Optional[int] = None):
-        """Layers `start .. stop` over the hidden states `x [B,L,D]` (no final norm)."""
+    def run_layers(self, x: torch.Tensor, mask: torch.Tensor, start: int = 0, stop: Optional[int] = None,
+                   w_static: bool = False):
+        """Layers `start .. stop` over the hidden states `x [B,L,D]` (no final norm).
+        `w_static`: behind the stack's own embedding lookup, no launch in flight writes
+        the weights."""
         c, p = self.cfg, self.p
         H = c.num_attention_heads
         hd = c.hidden_size // H
@@ -250,17 +257,17 @@ class ModernBertEncoder:
             is_global = li % c.global_attn_every_n_layers == 0
             cos, sin = tables[is_global]
             xn = x if lp["attn_ln_w"] is None else ops.layer_norm(x, lp["attn_ln_w"], None, c.norm_eps)
-            qkv = ops.linear(xn, lp["qkv_w"], Linear(rope=Rotary(cos, sin, 2 * H, hd)))
+            qkv = ops.linear(xn, lp["qkv_w"], Linear(rope=Rotary(cos, sin, 2 * H, hd), w_static=w_static))
             a = ops.attention_packed(qkv, H, H, Attn(keys=keys, window=None if is_global else (half, half)))
-            h = ops.linear(a.view(B, L, D), lp["o_w"], Linear(residual=x))
+            h = ops.linear(a.view(B, L, D), lp["o_w"], Linear(residual=x, w_static=w_static))
             hn = ops.layer_norm(h, lp["mlp_ln_w"], None, c.norm_eps)
-            g = ops.linear(hn, lp["wi_w"], Linear(act=Act.GELU, gated=True))
-            x = ops.linear(g, lp["wo_w"], Linear(residual=h))
+            g = ops.linear(hn, lp["wi_w"], Linear(act=Act.GELU, gated=True, w_static=w_static))
+            x = ops.linear(g, lp["wo_w"], Linear(residual=h, w_static=w_static))
         return x
 
     def forward(self, ids, mask, out=None, gather=None):
         c, p = self.cfg, self.p
-        x = self.run_layers(ops.embed_norm(ids, p["embed"], p["emb_ln_w"], None, c.norm_eps), mask)
+        x = self.run_layers(ops.embed_norm(ids, p["embed"], p["emb_ln_w"], None, c.norm_eps), mask, w_static=True)
         mode = ops.POOL_CLS if c.pooling == "cls" else ops.POOL_MEAN
         # final LayerNorm (of the tokens that are pooled), pooling and L2: one kernel
         return ops.norm_pool(x, p["final_ln_w"], None, c.norm_eps, aux=mask if mode == ops.POOL_MEAN else None,

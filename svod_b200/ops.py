@@ -72,6 +72,9 @@ class Linear:
     # None = this module's choice (`auto_k_splits`: one piece), 0 / 1 = the k loop in one
     # piece, > 1 = that many pieces on the CTA-pair kernel. The f32 workspace is allocated here.
     k_splits: Optional[int] = None
+    # No launch that may still be in flight writes `w` (a model's weights): the kernel may
+    # request its first tiles before the previous kernel of the stream has finished.
+    w_static: bool = False
 
 
 @dataclass
@@ -235,7 +238,7 @@ def linear(x: torch.Tensor, w: torch.Tensor, opts: Optional[Linear] = None) -> t
     keep = [_desc(opts.bias), _desc(opts.residual),
             _desc(opts.rope.cos) if opts.rope else None, _desc(opts.rope.sin) if opts.rope else None]
     o.bias = C.pointer(keep[0]) if keep[0] is not None else None
-    o.act = int(opts.act)
+    o.act = int(opts.act) | (L.LINEAR_W_STATIC if opts.w_static else 0)
     o.gated = int(opts.gated)
     o.residual = C.pointer(keep[1]) if keep[1] is not None else None
     o.has_scale = int(opts.scale is not None)
