@@ -769,7 +769,7 @@ int attend(const char* OP, const svodb_tensor* q, const svodb_tensor* k, const s
   }
   if (D > 256) return fail(SVODB_ERR_UNSUPPORTED, "%s: head dim %lld is above 256", OP, (long long)D);
   const char* why = !is_half(a.dtype) ? "dtype" : "shape";
-  int rc = launch_attention_generic(a, s);
+  int rc = attention_f32_covers(a) ? launch_attention_f32(a, s) : launch_attention_generic(a, s);
   if (rc != 0) return fail(SVODB_ERR_LAUNCH, "%s: kernel attributes were rejected (%d)", OP, rc);
   merge_splits();
   chose_graph(OP, why);

@@ -148,6 +148,9 @@ struct AttnArgs {
 };
 // Exact CUDA-core path (any float dtype, any D <= 256, every mask, bias, splits).
 int launch_attention_generic(const AttnArgs& a, cudaStream_t s);
+// The same for f32 operands on the 16-byte grid: register-tiled (attention_f32.cu).
+int launch_attention_f32(const AttnArgs& a, cudaStream_t s);
+bool attention_f32_covers(const AttnArgs& a);
 // tcgen05 path; returns 0 when it ran, nonzero (and launches nothing) when the
 // shape is outside what it covers.
 int launch_attention_tc(const AttnArgs& a, cudaStream_t s, char* cfg, size_t cfg_len);

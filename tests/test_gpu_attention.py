@@ -677,3 +677,27 @@ def test_few_query_rows_on_many_keys(B, T, Tk, H, Hkv, D, appended, mask):
             ref = np.log(np.exp(s - s.max(-1, keepdims=True)).sum(-1)) + s.max(-1)
         seen = ~np.isnan(ref)
         assert np.abs(host(out[1])[seen] - ref[seen]).max() < 1e-3 and np.all(np.isneginf(host(out[1])[~seen]))
+
+
+F32_CASES = [
+    # B, T, Tk, H, Hkv, D, kwargs: 64-row tiles, keys shared over clusters of 1..8
+    (1, 16, 1000, 2, 2, 64, dict(lens=[999])),            # eight shares, the last short
+    (1, 64, 64, 1, 1, 128, dict()),                       # one whole tile
+    (2, 65, 129, 4, 2, 36, dict(causal=True)),            # one row and one key past a tile, zero-filled columns
+    (2, 130, 200, 2, 2, 128, dict(lens=[0, 77])),         # a lane without keys
+    (2, 200, 200, 2, 1, 64, dict(window=(20, 5))),        # rows whose first tile lies past key 0
+    (40, 70, 70, 4, 4, 64, dict(mask="km")),              # more tiles than the chip holds, holes
+]
+
+
+@pytest.mark.parametrize("B,T,Tk,H,Hkv,D,kw", F32_CASES)
+def test_f32_attention_tiles_and_shares(B, T, Tk, H, Hkv, D, kw):
+    """Output and log-sum-exp of the f32 tile kernel within 1e-4 of the f64 oracle."""
+    kw = dict(kw)
+    if kw.get("mask") == "km":
+        kw["mask"] = key_mask(B, Tk)
+    rng = np.random.default_rng(B + T + Tk)
+    q, k, v = (O.round_to(O.F32, rng.standard_normal(s)) for s in ((B, T, H, D), (B, Tk, Hkv, D), (B, Tk, Hkv, D)))
+    got, glse, want, wlse = run_case(q, k, v, O.F32, lse=True, **kw)
+    assert ops.chosen() == "attention: graph dtype"
+    assert np.isfinite(got).all() and max_abs(got, want) < 1e-4 and max_abs(glse, wlse) < 1e-4
