@@ -233,6 +233,30 @@ SYMBOLS = [
 _lib = None
 
 
+_fast = None
+
+
+def fastops():
+    """The compiled call path (csrc/fastops.cpp), bound to this library's entry points."""
+    global _fast
+    if _fast is None:
+        import importlib.machinery
+        import importlib.util
+
+        import torch  # noqa: F401 — its libraries carry the symbols the module uses
+        path = Path(__file__).resolve().parent / "lib" / "_fastops.so"
+        if not path.exists():
+            raise RuntimeError(f"{path} is missing: build it with `python -m svod_b200.build`")
+        loader = importlib.machinery.ExtensionFileLoader("_fastops", str(path))
+        mod = importlib.util.module_from_spec(importlib.util.spec_from_file_location("_fastops", str(path), loader=loader))
+        loader.exec_module(mod)
+        lib = load()
+        mod.init(*[C.cast(getattr(lib, f"svodb_{n}"), C.c_void_p).value for n in (
+            "linear", "attention", "attention_packed", "layer_norm", "rms_norm", "add_layer_norm", "add_rms_norm")])
+        _fast = mod
+    return _fast
+
+
 def load() -> C.CDLL:
     """Loads the library once and types every entry point."""
     global _lib

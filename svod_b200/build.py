@@ -18,6 +18,7 @@ INCLUDE = ROOT.parent / "include"
 OUT_DIR = ROOT / "lib"
 OBJ_DIR = OUT_DIR / "obj"
 LIB = OUT_DIR / "libsvodb.so"
+FAST = OUT_DIR / "_fastops.so"  # the op layer's Python call path (csrc/fastops.cpp)
 
 NVCC = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")
 FLAGS = [
@@ -50,11 +51,33 @@ def _compile(src: Path, verbose: bool) -> Path:
     return obj
 
 
+def _build_fast() -> None:
+    """The CPython module against torch's headers; its torch symbols are those of the
+    libraries `import torch` has loaded."""
+    src = CSRC / "fastops.cpp"
+    stamp = max(src.stat().st_mtime, (INCLUDE / "svodb.h").stat().st_mtime)
+    if FAST.exists() and FAST.stat().st_mtime >= stamp:
+        return
+    import sysconfig
+
+    import torch
+    inc = Path(torch.__file__).resolve().parent / "include"
+    cmd = ["g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-w", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+           f"-I{INCLUDE}", f"-I{inc}", f"-I{inc}/torch/csrc/api/include", f"-I{sysconfig.get_paths()['include']}",
+           f"-I{Path(NVCC).parent.parent}/include", str(src), "-o", str(FAST), f"-L{inc.parent}/lib", "-ltorch_python", "-ltorch_cpu",
+           "-lc10", "-lc10_cuda"]
+    r = subprocess.run(cmd, capture_output=True, text=True)
+    if r.returncode != 0:
+        raise RuntimeError(f"g++ failed for {src.name}:\n{r.stdout}\n{r.stderr}")
+
+
 def build(verbose: bool = False) -> Path:
     OBJ_DIR.mkdir(parents=True, exist_ok=True)
     srcs = sorted(CSRC.glob("*.cu"))
-    with ThreadPoolExecutor(max_workers=min(8, len(srcs))) as ex:
+    with ThreadPoolExecutor(max_workers=min(8, len(srcs) + 1)) as ex:
+        fast = ex.submit(_build_fast)
         objs = list(ex.map(lambda s: _compile(s, verbose), srcs))
+    fast.result()
     if not LIB.exists() or any(o.stat().st_mtime > LIB.stat().st_mtime for o in objs):
         cmd = [NVCC, "-shared", "-gencode", "arch=compute_100a,code=sm_100a", "-o", str(LIB), *map(str, objs)]
         r = subprocess.run(cmd, capture_output=True, text=True)

@@ -175,6 +175,18 @@ def _stream() -> int:
     return torch.cuda.current_stream().cuda_stream
 
 
+def _fast():
+    """The compiled call path; the first call replaces this function's value in `_call`."""
+    global _call
+    _call = L.fastops()
+    return _call
+
+
+# The compiled forms of linear, attention and the norms (csrc/fastops.cpp): they return None,
+# with nothing launched, for any call out of the ordinary, which then takes the general
+# path below (and is converted or reported there).
+_call = None
+
 # Kernel launches issued through this module since import (an op that runs two
 # kernels, e.g. pooling + L2 or a split attention + merge, counts both).
 launches = 0
@@ -221,6 +233,11 @@ def auto_k_splits(m: int, n: int, k: int, opts: "Linear", dtype) -> int:
 def linear(x: torch.Tensor, w: torch.Tensor, opts: Optional[Linear] = None) -> torch.Tensor:
     """`ops::linear` (tk/src/ops/linear.rs:63-191): `x [lead..., K] . w [N, K]^T`
     with the epilogue `opts`."""
+    global launches
+    y = (_call or _fast()).linear(x, w, opts)
+    if y is not None:
+        launches += 1
+        return y
     opts = opts or Linear()
     lib = L.load()
     if w.dim() != 2:
@@ -331,9 +348,27 @@ def _attn_opts(opts: Attn, q_shape, dtype, device, keep: list):
     return o, lse
 
 
+_tune = None  # the tune module, once something has imported it
+
+
+def _tune_idle() -> bool:
+    """Whether no tune store would be asked for a split count."""
+    global _tune
+    if _tune is None:
+        from . import tune
+        _tune = tune
+    return _tune.active() is None
+
+
 def attention(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, opts: Optional[Attn] = None):
     """`ops::attention` (tk/src/ops/attention.rs:100-102): `q [B,T,H,D]`,
     `k,v [B,Tk,Hkv,D]` -> `[B,T,H,D]` (and `lse` when `opts.want_lse`)."""
+    global launches
+    if _tune_idle():
+        r = (_call or _fast()).attention(q, k, v, opts)
+        if r is not None:
+            launches += 1
+            return r
     opts = opts or Attn()
     if q.dim() != 4:
         raise OpsError(L.ERR_SHAPE, f"attention: q has shape {list(q.shape)}, expected [B, T, H, D]")
@@ -357,6 +392,11 @@ def attention(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, opts: Optional[
 def attention_packed(qkv: torch.Tensor, heads: int, kv_heads: int, opts: Optional[Attn] = None):
     """`ops::attention_packed` (tk/src/ops/attention.rs:107-122): the kernel
     reads q, k and v in place from `qkv [B, T, (heads + 2 kv_heads) D]`."""
+    global launches
+    r = (_call or _fast()).attention_packed(qkv, heads, kv_heads, opts)
+    if r is not None:
+        launches += 1
+        return r
     opts = opts or Attn()
     if kv_heads <= 0 or heads % kv_heads != 0:
         raise OpsError(L.ERR_HEADS, f"attention: {heads} query heads are not a multiple of {kv_heads} key/value heads")
@@ -414,6 +454,11 @@ def heads(qkv: torch.Tensor, opts: Qkv):
 # ---------------------------------------------------------------------------- norms
 def layer_norm(x, w, b=None, eps: float = 1e-5):
     """`ops::layer_norm` (tk/src/ops/norm.rs:17-19)."""
+    global launches
+    r = (_call or _fast()).norm(x, None, w, b, eps, True)
+    if r is not None:
+        launches += 1
+        return r
     out = torch.empty_like(x)
     xd, wd, bd, od = _desc(x), _desc(w), _desc(b), _desc(out)
     _check(L.load().svodb_layer_norm(_p(xd), _p(wd), _p(bd), float(eps), _p(od), _stream()))
@@ -422,6 +467,11 @@ def layer_norm(x, w, b=None, eps: float = 1e-5):
 
 def add_layer_norm(x, residual, w, b=None, eps: float = 1e-5):
     """`ops::add_layer_norm` (tk/src/ops/norm.rs:22-32): `(x + residual, norm)`."""
+    global launches
+    r = (_call or _fast()).norm(x, residual, w, b, eps, True)
+    if r is not None:
+        launches += 1
+        return r
     out, s = torch.empty_like(x), torch.empty_like(x)
     xd, rd, wd, bd, sd, od = _desc(x), _desc(residual), _desc(w), _desc(b), _desc(s), _desc(out)
     _check(L.load().svodb_add_layer_norm(_p(xd), _p(rd), _p(wd), _p(bd), float(eps), _p(sd), _p(od), _stream()))
@@ -430,6 +480,11 @@ def add_layer_norm(x, residual, w, b=None, eps: float = 1e-5):
 
 def rms_norm(x, w, eps: float = 1e-6):
     """`ops::rms_norm` (tk/src/ops/norm.rs:35-37)."""
+    global launches
+    r = (_call or _fast()).norm(x, None, w, None, eps, False)
+    if r is not None:
+        launches += 1
+        return r
     out = torch.empty_like(x)
     xd, wd, od = _desc(x), _desc(w), _desc(out)
     _check(L.load().svodb_rms_norm(_p(xd), _p(wd), float(eps), _p(od), _stream()))
@@ -438,6 +493,11 @@ def rms_norm(x, w, eps: float = 1e-6):
 
 def add_rms_norm(x, residual, w, eps: float = 1e-6):
     """`ops::add_rms_norm` (tk/src/ops/norm.rs:40-43): `(x + residual, norm)`."""
+    global launches
+    r = (_call or _fast()).norm(x, residual, w, None, eps, False)
+    if r is not None:
+        launches += 1
+        return r
     out, s = torch.empty_like(x), torch.empty_like(x)
     xd, rd, wd, sd, od = _desc(x), _desc(residual), _desc(w), _desc(s), _desc(out)
     _check(L.load().svodb_add_rms_norm(_p(xd), _p(rd), _p(wd), float(eps), _p(sd), _p(od), _stream()))
