@@ -319,6 +319,28 @@ int svodb_norm_pool(const svodb_tensor* hidden, const svodb_tensor* norm_w, cons
                     int32_t layer, svodb_tensor* scratch, const svodb_tensor* mask_or_lengths, int32_t mode,
                     int32_t normalize, svodb_tensor* out, void* stream);
 
+/* Packed rows: a padded batch [B, L] computed without its trailing padding. No
+ * counterpart in the reference, which computes every padded position.
+ * `svodb_rows_begin` launches the kernel that works the layout out from the padding
+ * mask [B, L] (u8 / i32) or the lengths [B] (i32) and turns it on for the calling
+ * thread; until `svodb_rows_end` every op of this thread (on the same stream) takes
+ * and makes tensors [B, L', ...], L' = L rounded up to 64, that hold the packed rows
+ * one after the other: batch row b is cut after its last real token, rounded up to
+ * whole 64-position blocks (one block at least), and what lies behind the last packed
+ * row is undefined. `svodb_embed(_norm)` puts ids [B, L] into that form,
+ * `svodb_norm_pool(_gather)` (CLS, mean, last token) reads it back out; between them
+ * `svodb_linear`, the norms and `svodb_attention_packed` run on it. Key masks are
+ * [B, L']: `mask_out` (bytes; NULL without a mask) receives the mask in that form.
+ * Rotation tables have L' rows. `table`: `svodb_rows_table_bytes` bytes of device
+ * memory, zero before its first use and kept until the ops are done; one use at a time.
+ * SVODB_ERR_UNSUPPORTED from any of these ops means that this call has no kernel over
+ * packed rows: end them and run the padded form. */
+size_t svodb_rows_table_bytes(int64_t batch, int64_t len);
+/* Whether the library's own stacks run a plan [batch, len] that way. */
+int svodb_rows_pay(int64_t batch, int64_t len);
+int svodb_rows_begin(const svodb_tensor* mask_or_lengths, int64_t len, void* table, svodb_tensor* mask_out, void* stream);
+void svodb_rows_end(void);
+
 /* RoPE tables `Tensor::rope_table` (tensor/src/transformer.rs:130-164): angles
  * and cos/sin in f32, cast last; positions [P] i32 (NULL = 0..P-1);
  * cos,sin [P, head_dim/2]. */

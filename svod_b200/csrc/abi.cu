@@ -171,6 +171,22 @@ bool same_shape(const svodb_tensor* a, const svodb_tensor* b) {
   return true;
 }
 
+// The row layout this thread's ops run under (`svodb_rows_begin` .. `svodb_rows_end`).
+struct ActiveRows {
+  bool on;
+  RowLayout layout;
+};
+thread_local ActiveRows g_rows{};
+
+// The layout in force, or null. Operands under one are the packed rows of [B, L rounded up, ...].
+const RowLayout* active_rows() { return g_rows.on ? &g_rows.layout : nullptr; }
+bool rows_fit(const svodb_tensor* t) {
+  return t->rank >= 3 && t->shape[0] == g_rows.layout.batch && t->shape[1] == g_rows.layout.len;
+}
+int rows_unsupported(const char* op) {
+  return fail(SVODB_ERR_UNSUPPORTED, "%s: this call does not run over packed rows", op);
+}
+
 #define TRY(expr)                  \
   do {                             \
     int rc_ = (expr);              \
@@ -431,6 +447,14 @@ int svodb_linear(const svodb_tensor* x, const svodb_tensor* w, const svodb_linea
   a.dtype = x->dtype;
   a.status = device_status_word();
   a.w_static = (opts->act & SVODB_LINEAR_W_STATIC) != 0;
+  const RowLayout* rows = active_rows();
+  if (rows != nullptr) {
+    if (!rows_fit(x)) return shape_err(OP, "x", x, "[B, L, K] of the packed rows");
+    if (qkv_per_batch) return rows_unsupported(OP);
+    a.live = rows->live, a.block_pos = rows->block_pos;
+  }
+  // position-dependent stores only the tensor-core kernels find the way to under packed rows
+  const bool placed = rows != nullptr && (rope || (qo != nullptr && (qo->rope_cos != nullptr || qo->q_norm != nullptr || qo->k_norm != nullptr)));
   if (a.m == 0 || n == 0) {
     chose_graph(OP, "shape");
     return SVODB_OK;
@@ -501,6 +525,7 @@ int svodb_linear(const svodb_tensor* x, const svodb_tensor* w, const svodb_linea
         return check_launch(OP);
       }
     }
+    if (any && placed) return rows_unsupported(OP);
     if (any && !contiguous(y))
       return fail(SVODB_ERR_GRAPH, "%s: the qkv prologue outside the kernel needs a contiguous y", OP);
   }
@@ -551,6 +576,7 @@ int svodb_linear(const svodb_tensor* x, const svodb_tensor* w, const svodb_linea
       return check_launch(OP);
     }
   }
+  if (placed) return rows_unsupported(OP);
   const char* why = !is_half(a.dtype) ? "dtype" : (n % 8 != 0 || k % 16 != 0) ? "shape" : "config";
   launch_gemm_generic(a, s);
   if (qo != nullptr) heads_in_place(qo, y, qkv_per_batch, s);
@@ -701,6 +727,16 @@ int attend(const char* OP, const svodb_tensor* q, const svodb_tensor* k, const s
   a.splits = opts->splits > 1 ? opts->splits : 1;
   a.status = device_status_word();
   a.packed = packed;
+  const bool exact_only = config_lookup("attention|exact") != 0;
+  const bool one_item = config_lookup("attention|one_item") != 0;
+  const RowLayout* rows = active_rows();
+  if (rows != nullptr) {
+    if (!rows_fit(q)) return shape_err(OP, "q", q, "[B, L, H, D] of the packed rows");
+    a.layout = rows;
+    if (!packed || !contiguous(o) || opts->seg_start != nullptr || opts->bias != nullptr || opts->lse != nullptr ||
+        opts->splits > 1 || exact_only || one_item || !attention_tc_p_covers(a))
+      return rows_unsupported(OP);
+  }
   if (B * T * H == 0 || D == 0) {
     chose_graph(OP, "shape");
     return SVODB_OK;
@@ -740,9 +776,7 @@ int attend(const char* OP, const svodb_tensor* q, const svodb_tensor* k, const s
     c.dtype = a.dtype;
     launch_combine(c, s);
   };
-  const bool exact_only = config_lookup("attention|exact") != 0;
-  const bool one_item = config_lookup("attention|one_item") != 0;
-  if (!exact_only && !one_item && attention_decode_covers(a)) {
+  if (rows == nullptr && !exact_only && !one_item && attention_decode_covers(a)) {
     int rc = launch_attention_decode(a, s, cfg, sizeof cfg);
     if (rc < 0) return fail(SVODB_ERR_LAUNCH, "%s: the tensor map or kernel attributes were rejected", OP);
     if (rc == 0) {
@@ -759,6 +793,7 @@ int attend(const char* OP, const svodb_tensor* q, const svodb_tensor* k, const s
       return check_launch(OP);
     }
   }
+  if (rows != nullptr) return rows_unsupported(OP);
   if (!exact_only && attention_tc_covers(a)) {
     int rc = launch_attention_tc(a, s, cfg, sizeof cfg);
     if (rc < 0) return fail(SVODB_ERR_LAUNCH, "%s: the tensor map or kernel attributes were rejected", OP);
@@ -859,6 +894,53 @@ int svodb_combine_splits(const svodb_tensor* o_part, const svodb_tensor* m_part,
 }
 
 // ---------------------------------------------------------------------------
+// packed rows
+// ---------------------------------------------------------------------------
+size_t svodb_rows_table_bytes(int64_t batch, int64_t len) {
+  return batch > 0 && len > 0 ? sizeof(int32_t) * row_layout_ints(batch, len) : 0;
+}
+
+// Below 1024 padded rows a stack is bound by its launches, not by its rows.
+int svodb_rows_pay(int64_t batch, int64_t len) { return batch > 0 && len > 0 && batch * len >= 1024 ? 1 : 0; }
+
+int svodb_rows_begin(const svodb_tensor* mask_or_lengths, int64_t len, void* table, svodb_tensor* mask_out, void* stream) {
+  static const char* OP = "rows_begin";
+  GUARD(OP);
+  const svodb_tensor* aux = mask_or_lengths;
+  TRY(realized(OP, "mask or lengths", aux));
+  if (g_rows.on) return fail(SVODB_ERR_GRAPH, "%s: this thread already runs over packed rows", OP);
+  if (table == nullptr) return fail(SVODB_ERR_WORKSPACE, "%s: the table is missing", OP);
+  const bool mask = aux->rank == 2;
+  if (!(aux->rank == 1 || (mask && aux->shape[1] == len)) || aux->shape[0] <= 0 || len <= 0 || !contiguous(aux))
+    return shape_err(OP, "mask or lengths", aux, "[B, L] or [B]");
+  if (aux->dtype != SVODB_I32 && !(mask && aux->dtype == SVODB_U8))
+    return dtype_err(OP, "mask or lengths", aux->dtype, mask ? SVODB_U8 : SVODB_I32);
+  const int64_t B = aux->shape[0], padded = (len + kRowBlock - 1) / kRowBlock * kRowBlock;
+  if (B * padded > 0x7fffffffLL) return rows_unsupported(OP);
+  if (mask_out != nullptr) {
+    TRY(realized(OP, "mask out", mask_out));
+    if (!mask || mask_out->rank != 2 || mask_out->shape[0] != B || mask_out->shape[1] != padded || !contiguous(mask_out) ||
+        mask_out->dtype != SVODB_U8)
+      return shape_err(OP, "mask out", mask_out, "[B, L rounded up to 64] bytes beside a mask");
+    TRY(no_alias(OP, mask_out, {aux}));
+  }
+  if (!attention_tc_p_ready((cudaStream_t)stream)) return rows_unsupported(OP);
+  RowLayoutArgs a{};
+  if (mask) a.mask = aux->data, a.mask_i32 = aux->dtype == SVODB_I32;
+  else a.lengths = (const int32_t*)aux->data;
+  a.batch = B, a.len = len;
+  a.table = (int32_t*)table;
+  a.mask_out = mask_out != nullptr ? (uint8_t*)mask_out->data : nullptr;
+  launch_row_layout(a, (cudaStream_t)stream);
+  TRY(check_launch(OP));
+  g_rows.layout = row_layout_of(B, len, a.table);
+  g_rows.on = true;
+  return SVODB_OK;
+}
+
+void svodb_rows_end(void) { g_rows.on = false; }
+
+// ---------------------------------------------------------------------------
 // heads
 // ---------------------------------------------------------------------------
 int svodb_heads(const svodb_tensor* qkv, const svodb_qkv_opts* opts, svodb_tensor* q, svodb_tensor* k,
@@ -910,6 +992,7 @@ int svodb_heads(const svodb_tensor* qkv, const svodb_qkv_opts* opts, svodb_tenso
   TRY(no_alias(OP, q, {qkv, k, v}));
   TRY(no_alias(OP, k, {qkv, v}));
   TRY(no_alias(OP, v, {qkv}));
+  if (active_rows() != nullptr) return rows_unsupported(OP);
   HeadsArgs a{};
   a.qkv = qkv->data;
   a.q_w = opts->q_norm ? opts->q_norm->data : nullptr;
@@ -971,6 +1054,10 @@ int norm_op(const char* OP, int layer, const svodb_tensor* x, const svodb_tensor
   a.eps = (float)eps;
   a.layer = layer;
   a.dtype = x->dtype;
+  if (active_rows() != nullptr) {
+    if (!rows_fit(x)) return shape_err(OP, "x", x, "[B, L, D] of the packed rows");
+    a.live = g_rows.layout.live;
+  }
   if (a.rows == 0) {
     chose_graph(OP, "shape");
     return SVODB_OK;
@@ -1029,7 +1116,11 @@ int embed_impl(const char* OP, const svodb_tensor* ids, const svodb_tensor* tabl
   if (!is_half(table->dtype)) return dtype_err(OP, "table", table->dtype, SVODB_BF16);
   const int64_t d = table->shape[1];
   if (d % 8 != 0) return shape_err(OP, "table", table, "[V, D] with D a multiple of 8");
-  if (out->rank != 3 || out->shape[0] != ids->shape[0] || out->shape[1] != ids->shape[1] || out->shape[2] != d ||
+  const RowLayout* rows = active_rows();
+  const int64_t out_len = rows != nullptr ? rows->len : ids->shape[1];
+  if (rows != nullptr && (ids->shape[0] != rows->batch || (ids->shape[1] + kRowBlock - 1) / kRowBlock * kRowBlock != rows->len))
+    return shape_err(OP, "ids", ids, "[B, L] of the packed rows");
+  if (out->rank != 3 || out->shape[0] != ids->shape[0] || out->shape[1] != out_len || out->shape[2] != d ||
       !contiguous(out) || out->dtype != table->dtype)
     return shape_err(OP, "out", out, "[B, T, D]");
   if (pos_table != nullptr) {
@@ -1053,6 +1144,7 @@ int embed_impl(const char* OP, const svodb_tensor* ids, const svodb_tensor* tabl
   a.d = (int)d;
   a.vocab = table->shape[0];
   a.max_pos = pos_table ? pos_table->shape[0] : 1;
+  a.layout = rows;
   a.dtype = table->dtype;
   if (norm_w == nullptr) {
     launch_embed(a, (cudaStream_t)stream);
@@ -1068,7 +1160,7 @@ int embed_impl(const char* OP, const svodb_tensor* ids, const svodb_tensor* tabl
   launch_embed(a, (cudaStream_t)stream);
   NormArgs r{};
   r.x = out->data, r.w = norm_w->data, r.b = n.b, r.out = out->data;
-  r.rows = a.batch * a.t, r.d = a.d, r.eps = n.eps, r.layer = layer, r.dtype = a.dtype;
+  r.rows = a.batch * out_len, r.d = a.d, r.live = rows != nullptr ? rows->live : nullptr, r.eps = n.eps, r.layer = layer, r.dtype = a.dtype;
   launch_norm(r, (cudaStream_t)stream);
   chose_graph(OP, "shape");
   return check_launch(OP);
@@ -1120,6 +1212,11 @@ int pool_impl(const char* OP, const svodb_tensor* hidden, const svodb_tensor* no
     if (aux->dtype != SVODB_I32) return dtype_err(OP, "lengths", aux->dtype, SVODB_I32);
   }
   if (L == 0) return shape_err(OP, "hidden", hidden, "[B, L >= 1, D]");
+  const RowLayout* rows = active_rows();
+  if (rows != nullptr) {
+    if (!rows_fit(hidden)) return shape_err(OP, "hidden", hidden, "[B, L, D] of the packed rows");
+    if (!fused || mode == 3) return rows_unsupported(OP);
+  }
   PoolArgs a{};
   a.push = push;
   a.hidden = hidden->data;
@@ -1133,6 +1230,10 @@ int pool_impl(const char* OP, const svodb_tensor* hidden, const svodb_tensor* no
   a.batch = B, a.l = L;
   a.d = (int)D;
   a.dtype = hidden->dtype;
+  if (rows != nullptr) {
+    a.row_start = rows->start;
+    if (mode == 2) a.aux = rows->keys;  // the lengths, cut to L as the layout cut them
+  }
   if (!fused) {
     launch_pool(a, (cudaStream_t)stream);
     return check_launch(OP);
@@ -1145,6 +1246,7 @@ int pool_impl(const char* OP, const svodb_tensor* hidden, const svodb_tensor* no
                                          : (push != nullptr && push->world > 1 ? "{norm:none,push:peers}" : "{norm:none}"));
     return check_launch(OP);
   }
+  if (rows != nullptr) return rows_unsupported(OP);
   a.push = nullptr;  // the unfused kernels below do not send
   // outside the fused kernel's rows: the norm into the caller's scratch, then the two pooling kernels
   if (norm_w != nullptr) {

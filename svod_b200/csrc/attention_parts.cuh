@@ -41,6 +41,12 @@ struct FaParams {
   int has_chunk;
   int64_t chunk_size, chunk_left, chunk_right;
   const int32_t* seg_start;
+  // packed rows (persistent kernel): per batch lane the first row, the query rows, the visible keys
+  // and whether the key mask has holes before them; q, k, v and o are then one lane of all rows
+  const int32_t* row_start;
+  const int32_t* row_count;
+  const int32_t* row_keys;
+  const int32_t* row_holes;
   const int32_t* row_map;  // `ops::Cache`: cache row of batch lane b, or null
   float* lse;
   int n_qt;  // work items per (head or head pair, batch): pairs of 128-row tiles, or 128-row tiles when pair_heads
@@ -77,10 +83,10 @@ struct Ctx {
   int general_mask;  // the key mask is not a prefix: consult the bitmask
 };
 
-__device__ __forceinline__ Range tile_range(const FaParams& p, const Ctx& c, int64_t b, int64_t i_first) {
+__device__ __forceinline__ Range tile_range(const FaParams& p, const Ctx& c, int64_t b, int64_t i_first, int64_t t) {
   Range r{0, 0};
-  if (i_first >= p.t) return r;
-  const int64_t i_last = (i_first + kBQ - 1 < p.t - 1) ? i_first + kBQ - 1 : p.t - 1;
+  if (i_first >= t) return r;
+  const int64_t i_last = (i_first + kBQ - 1 < t - 1) ? i_first + kBQ - 1 : t - 1;
   int64_t lo = 0, hi = c.len;
   if (p.causal && i_last + 1 < hi) hi = i_last + 1;
   if (p.has_window) {

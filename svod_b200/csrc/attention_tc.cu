@@ -169,8 +169,8 @@ __global__ void __launch_bounds__(kThreadsFa, 1)
     if (first_zero < last_set) ctx.general_mask = 1;  // not a prefix: consult the bitmask
     if (last_set < ctx.len) ctx.len = last_set;
   }
-  const Range r0 = tile_range(p, ctx, b, i0);
-  const Range r1 = tile_range(p, ctx, b, i0 + kBQ);
+  const Range r0 = tile_range(p, ctx, b, i0, p.t);
+  const Range r1 = tile_range(p, ctx, b, i0 + kBQ, p.t);
   const bool live0 = r0.hi > r0.lo, live1 = r1.hi > r1.lo;
   int u_lo = 0, u_hi = 0;
   if (live0 && live1) {

@@ -159,6 +159,8 @@ struct Work {
   int len, general;  // the mask context (`Ctx`): visible key bound, whether to consult the bitmask
   Range r0, r1;
   int u_lo, u_hi;    // the union of the two ranges: the blocks the loader brings
+  int t;             // query rows of the batch lane
+  int tb, base;      // where the lane lies in the tensors: batch coordinate, first row (packed rows: 0 and its start)
 };
 
 // The read-out of one tile's O by one softmax warp (32 rows): 64 columns at a time
@@ -280,6 +282,7 @@ __global__ void __launch_bounds__(kThreadsFa, 1)
     w.hk = w.h / (p.heads / p.kv_heads);
     w.b = it.b;
     w.i0 = it.qt * (p.pair_heads ? kBQ : 2 * kBQ);
+    w.t = (int)p.t, w.tb = it.b, w.base = 0;
     Ctx ctx;
     ctx.len = p.tk;
     ctx.general_mask = 0;
@@ -291,10 +294,14 @@ __global__ void __launch_bounds__(kThreadsFa, 1)
       ctx.general_mask = mrow.general;
       if (mrow.len < ctx.len) ctx.len = mrow.len;
     }
+    if (p.row_start != nullptr) {
+      w.t = p.row_count[it.b], w.tb = 0, w.base = p.row_start[it.b];
+      if (p.row_keys[it.b] < ctx.len) ctx.len = p.row_keys[it.b];
+    }
     w.len = (int)ctx.len;
     w.general = ctx.general_mask;
-    w.r0 = tile_range(p, ctx, w.b, w.i0);
-    w.r1 = tile_range(p, ctx, w.b, (int64_t)w.i0 + (p.pair_heads ? 0 : kBQ));
+    w.r0 = tile_range(p, ctx, w.b, w.i0, w.t);
+    w.r1 = tile_range(p, ctx, w.b, (int64_t)w.i0 + (p.pair_heads ? 0 : kBQ), w.t);
     w.split = it.split;
     if (EXTRAS && p.splits > 1) {
       // this split's share of the key blocks
@@ -345,7 +352,11 @@ __global__ void __launch_bounds__(kThreadsFa, 1)
           // The loader alone scans a bool key mask row (all its lanes, once per change
           // of batch lane, while it runs ahead of the other warps) and hands what it
           // found to them with the item.
-          if (it.valid && p.key_mask != nullptr) scan_mask_row(p, it.b, lane, mrow);
+          // (packed rows bring it along.)
+          if (it.valid && p.key_mask != nullptr) {
+            if (p.row_start != nullptr) mrow = MaskRow{it.b, p.row_keys[it.b], p.row_holes[it.b]};
+            else scan_mask_row(p, it.b, lane, mrow);
+          }
           Work w{};
           if (it.valid) w = plan(it, mrow);
           if (lane == 0) {
@@ -367,10 +378,10 @@ __global__ void __launch_bounds__(kThreadsFa, 1)
               mbar_expect_tx(&q_full[i], QB);
               for (int c = 0; c < D / 64; ++c)
                 tma_load_4d(q_s + i * QB + c * (128 * 128), &tmap_q, &q_full[i], c * 64, w.h + (p.pair_heads ? i : 0),
-                            w.i0 + (p.pair_heads ? 0 : i * kBQ), w.b);
+                            w.base + w.i0 + (p.pair_heads ? 0 : i * kBQ), w.tb);
             }
           }
-          const int kv_b = p.row_map != nullptr ? p.row_map[w.b] : w.b;
+          const int kv_b = p.row_map != nullptr ? p.row_map[w.b] : w.tb;
           for (int j = w.u_lo; j < w.u_hi && ok; ++j) {
             if (!mbar_wait(&k_empty[s], ph ^ 1, p.status)) {
               ok = false;
@@ -378,14 +389,14 @@ __global__ void __launch_bounds__(kThreadsFa, 1)
             }
             mbar_expect_tx(&k_full[s], KB);
             for (int c = 0; c < D / 64; ++c)
-              tma_load_4d(k_s + s * KB + c * KBOX, &tmap_k, &k_full[s], c * 64, w.hk, j * kBKV, kv_b);
+              tma_load_4d(k_s + s * KB + c * KBOX, &tmap_k, &k_full[s], c * 64, w.hk, w.base + j * kBKV, kv_b);
             if (!mbar_wait(&v_empty[s], ph ^ 1, p.status)) {
               ok = false;
               break;
             }
             mbar_expect_tx(&v_full[s], KB);
             for (int c = 0; c < D / 64; ++c)
-              tma_load_4d(v_s + s * KB + c * KBOX, &tmap_v, &v_full[s], c * 64, w.hk, j * kBKV, kv_b);
+              tma_load_4d(v_s + s * KB + c * KBOX, &tmap_v, &v_full[s], c * 64, w.hk, w.base + j * kBKV, kv_b);
             if (++s == S) {
               s = 0;
               ph ^= 1;
@@ -545,10 +556,10 @@ __global__ void __launch_bounds__(kThreadsFa, 1)
       const int64_t b = w.b;
       const int64_t i_first = (int64_t)w.i0 + (p.pair_heads ? 0 : (int64_t)i * kBQ);
       const int64_t row = i_first + quarter * 32 + lane;
-      const bool row_ok = row < p.t;
-      const int64_t i_last = (i_first + kBQ - 1 < p.t - 1) ? i_first + kBQ - 1 : p.t - 1;
+      const bool row_ok = row < w.t;
+      const int64_t i_last = (i_first + kBQ - 1 < w.t - 1) ? i_first + kBQ - 1 : w.t - 1;
       int64_t seg_me = 0, seg_last = 0;
-      if (p.seg_start != nullptr && i_first < p.t) {
+      if (p.seg_start != nullptr && i_first < w.t) {
         seg_me = p.seg_start[b * p.t + (row_ok ? row : i_last)];
         seg_last = p.seg_start[b * p.t + i_last];
       }
@@ -755,7 +766,7 @@ __global__ void __launch_bounds__(kThreadsFa, 1)
         continue;
       }
       // ---- epilogue: O / l, or this split's unnormalised state ----
-      T* orow = (T*)p.o + b * p.o_sb + row * p.o_st + (int64_t)h * p.o_sh;
+      T* orow = (T*)p.o + w.tb * p.o_sb + (w.base + row) * p.o_st + (int64_t)h * p.o_sh;
       const int64_t prow = (((int64_t)w.split * p.batch + b) * p.t + row) * p.heads + h;  // partial-state row
       float* oprow = EXTRAS && p.splits > 1 ? p.o_part + prow * p.d_real : nullptr;
       if (nblk > 0) {
@@ -784,8 +795,8 @@ __global__ void __launch_bounds__(kThreadsFa, 1)
           }
         } else {
           const int64_t row0 = i_first + quarter * 32;
-          store_o_slab<T, D>(o_tmem, inv, o_stage + (warp - 4) * (32 * 128), lane, &tmap_o, h, (int)row0, (int)b,
-                             p.d_real, row0 < p.t);
+          store_o_slab<T, D>(o_tmem, inv, o_stage + (warp - 4) * (32 * 128), lane, &tmap_o, h, w.base + (int)row0, w.tb,
+                             p.d_real, row0 < w.t);
         }
         // O is read out: the next live item's first P.V may overwrite it
         tc_fence_before();
@@ -871,13 +882,16 @@ int run_p(const AttnArgs& a, cudaStream_t s, char* cfg, size_t cfg_len) {
   CUtensorMap tq, tk, tv;
   const uint32_t box[4] = {64, 1, 128, 1};
   const uint32_t kvbox[4] = {64, 1, kBKV, 1};
+  // packed rows: one lane of B * T rows
+  const bool packed = a.layout != nullptr;
+  const uint64_t t_rows = packed ? (uint64_t)(a.batch * a.t) : (uint64_t)a.t, t_batch = packed ? 1 : (uint64_t)a.batch;
   {
-    const uint64_t dims[4] = {(uint64_t)a.d, (uint64_t)a.heads, (uint64_t)a.t, (uint64_t)a.batch};
+    const uint64_t dims[4] = {(uint64_t)a.d, (uint64_t)a.heads, t_rows, t_batch};
     const uint64_t st[3] = {(uint64_t)a.q_sh, (uint64_t)a.q_st, (uint64_t)a.q_sb};
     if (!make_tmap(&tq, a.q, a.dtype, 4, dims, st, box)) return -1;
   }
   {
-    const uint64_t dims[4] = {(uint64_t)a.d, (uint64_t)a.kv_heads, (uint64_t)a.tk, (uint64_t)a.kv_rows};
+    const uint64_t dims[4] = {(uint64_t)a.d, (uint64_t)a.kv_heads, packed ? t_rows : (uint64_t)a.tk, packed ? 1 : (uint64_t)a.kv_rows};
     const uint64_t stk[3] = {(uint64_t)a.k_sh, (uint64_t)a.k_st, (uint64_t)a.k_sb};
     const uint64_t stv[3] = {(uint64_t)a.v_sh, (uint64_t)a.v_st, (uint64_t)a.v_sb};
     if (!make_tmap(&tk, a.k, a.dtype, 4, dims, stk, kvbox)) return -1;
@@ -887,7 +901,7 @@ int run_p(const AttnArgs& a, cudaStream_t s, char* cfg, size_t cfg_len) {
   if (a.o != nullptr) {
     // the output as 32-row x 64-column boxes, one per softmax warp and store
     const uint32_t obox[4] = {64, 1, 32, 1};
-    const uint64_t dims[4] = {(uint64_t)a.d, (uint64_t)a.heads, (uint64_t)a.t, (uint64_t)a.batch};
+    const uint64_t dims[4] = {(uint64_t)a.d, (uint64_t)a.heads, t_rows, t_batch};
     const uint64_t st[3] = {(uint64_t)a.o_sh, (uint64_t)a.o_st, (uint64_t)a.o_sb};
     if (!make_tmap(&to, a.o, a.dtype, 4, dims, st, obox)) return -1;
   }
@@ -919,6 +933,10 @@ int run_p(const AttnArgs& a, cudaStream_t s, char* cfg, size_t cfg_len) {
   p.has_chunk = a.has_chunk;
   p.chunk_size = a.chunk_size, p.chunk_left = a.chunk_left, p.chunk_right = a.chunk_right;
   p.seg_start = a.seg_start;
+  if (packed) {
+    p.row_start = a.layout->start, p.row_count = a.layout->rows;
+    p.row_keys = a.layout->keys, p.row_holes = a.layout->holes;
+  }
   p.row_map = a.row_map;
   p.lse = a.lse;
   p.pair_heads = pairs_heads(a) ? 1 : 0;
@@ -977,8 +995,10 @@ bool attention_tc_p_covers(const AttnArgs& a) {
       return false;
     return true;
   }
-  return items > 148;
+  return items > 148 || a.layout != nullptr;
 }
+
+bool attention_tc_p_ready(cudaStream_t s) { return queue_head(s) != nullptr; }
 
 int launch_attention_tc_p(const AttnArgs& a, cudaStream_t s, char* cfg, size_t cfg_len) {
   if (!attention_tc_p_covers(a)) return 1;

@@ -3,6 +3,7 @@
 #pragma once
 
 #include "common.cuh"
+#include "kernels.h"
 
 namespace svodb {
 namespace gemm_parts {
@@ -17,6 +18,17 @@ __device__ __forceinline__ void tile_coords(int t, int tiles_m, int tiles_n, int
   const int r = t - group * per_group;
   mt = first + r % gsize;
   nt = r / gsize;
+}
+
+// Tile rows to walk: all, or those of the packed rows (`live`, read after `pdl_wait`).
+__device__ __forceinline__ int live_tiles(const int32_t* live, int tiles_m, int tile_rows) {
+  if (live == nullptr) return tiles_m;
+  const int t = (*reinterpret_cast<const volatile int32_t*>(live) + tile_rows - 1) / tile_rows;
+  return t < tiles_m ? t : tiles_m;
+}
+// The rotation table row of row `row` of x.
+__device__ __forceinline__ int64_t table_row(int64_t row, int64_t rope_seq, const int32_t* block_pos) {
+  return block_pos != nullptr ? block_pos[row / kRowBlock] + row % kRowBlock : row % rope_seq;
 }
 
 template <typename T>

@@ -68,6 +68,7 @@ struct ParamsS {
   const void* rope_sin;
   int rope_width;
   int64_t rope_seq;
+  const int32_t* block_pos;  // packed rows: their blocks' positions, nullable
   uint32_t* status;
 };
 
@@ -303,7 +304,7 @@ __global__ void __launch_bounds__(kThreads, 2)
     uint4 c4 = zero, s4 = zero;
     const bool turned = col < p.rope_width;
     if (turned) {
-      const int64_t tab = (int64_t)((uint32_t)grow % (uint32_t)p.rope_seq) * (BN / 2) + (ch & (BN / 16 - 1)) * 8;
+      const int64_t tab = table_row((uint32_t)grow, p.rope_seq, p.block_pos) * (BN / 2) + (ch & (BN / 16 - 1)) * 8;
       c4 = ldg128((const T*)p.rope_cos + tab);
       s4 = ldg128((const T*)p.rope_sin + tab);
     }
@@ -387,6 +388,7 @@ int run_s(const GemmArgs& a, int splits, cudaStream_t s, char* cfg, size_t cfg_l
   p.ldr = a.ldr, p.ldc = a.ldc;
   p.w_static = a.w_static;
   p.status = a.status;
+  p.block_pos = a.block_pos;
   const bool per_head = a.rope_cos != nullptr || a.norm_q != nullptr || a.norm_k != nullptr;
   if (per_head) {
     p.head = BN;

@@ -82,6 +82,8 @@ struct Params {
   const void* norm_k;
   int norm_q_cols, norm_cols;
   float norm_eps;
+  const int32_t* live;       // nullable: packed rows to compute; tiles past them are not walked
+  const int32_t* block_pos;  // their blocks' positions
   uint32_t* status;
 };
 
@@ -133,7 +135,6 @@ __global__ void __launch_bounds__(kThreads, 1)
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
   const int num_kb = (p.k + BK - 1) / BK;
-  const int num_tiles = p.tiles_m * p.tiles_n;
 
   if (threadIdx.x == 0) {
     for (int i = 0; i < S; ++i) {
@@ -154,6 +155,8 @@ __global__ void __launch_bounds__(kThreads, 1)
     tmem_relinquish();
   }
   pdl_wait();
+  const int tiles_m = live_tiles(p.live, p.tiles_m, BM);
+  const int num_tiles = tiles_m * p.tiles_n;
   if ((p.head_epilogue || p.head64_epilogue) && threadIdx.x < 256) {
     const T* wsrc = (const T*)(threadIdx.x < 128 ? p.norm_q : p.norm_k);
     const int at = threadIdx.x & 127;
@@ -174,7 +177,7 @@ __global__ void __launch_bounds__(kThreads, 1)
       uint32_t issued = 0;
       for (int t = blockIdx.x; t < num_tiles && ok; t += gridDim.x) {
         int mt, nt;
-        tile_coords(t, p.tiles_m, p.tiles_n, mt, nt);
+        tile_coords(t, tiles_m, p.tiles_n, mt, nt);
         const int m0 = mt * BM;
         const int n0 = nt * p.out_bn;
         for (int kb = 0; kb < num_kb; ++kb) {
@@ -272,7 +275,7 @@ __global__ void __launch_bounds__(kThreads, 1)
     bool ok = true;
     for (int t = blockIdx.x; t < num_tiles && ok; t += gridDim.x) {
       int mt, nt;
-      tile_coords(t, p.tiles_m, p.tiles_n, mt, nt);
+      tile_coords(t, tiles_m, p.tiles_n, mt, nt);
       const int64_t row = (int64_t)mt * BM + quarter * 32 + lane;
       const bool row_ok = row < p.m;
       const int n0 = nt * p.out_bn;
@@ -283,7 +286,7 @@ __global__ void __launch_bounds__(kThreads, 1)
       // finish (the second half of each 128-byte table row then hits L1).
       uint4 cs4[4], sn4[4];
       const bool head_turned = p.head_epilogue && n0 + c_lo < p.rope_width;
-      const int64_t rope_pos = row_ok ? row % p.rope_seq : 0;
+      const int64_t rope_pos = row_ok ? table_row(row, p.rope_seq, p.block_pos) : 0;
       if (head_turned) {
 #pragma unroll
         for (int v = 0; v < 4; ++v) {
@@ -388,7 +391,7 @@ __global__ void __launch_bounds__(kThreads, 1)
         const int m0 = mt * BM;
         const T* cos = (const T*)p.rope_cos;
         const T* sin = (const T*)p.rope_sin;
-        const int64_t pos = row_ok ? row % p.rope_seq : 0;
+        const int64_t pos = row_ok ? table_row(row, p.rope_seq, p.block_pos) : 0;
         for (int sub = 0; sub < cols / 64; ++sub) {
           const int c0 = c_lo + sub * 64;
           const int h_col = n0 + c0;
@@ -584,7 +587,7 @@ __global__ void __launch_bounds__(kThreads, 1)
         const int hd = p.rope_head_dim, half = hd / 2;
         const T* cos = (const T*)p.rope_cos;
         const T* sin = (const T*)p.rope_sin;
-        const int64_t pos = row_ok ? row % p.rope_seq : 0;
+        const int64_t pos = row_ok ? table_row(row, p.rope_seq, p.block_pos) : 0;
         for (int h0 = c_lo; h0 < c_lo + cols; h0 += hd) {
           const bool turned = n0 + h0 < p.rope_width;
           for (int j = 0; j < half; j += 32) {
@@ -765,6 +768,7 @@ int launch_gemm_tc(const GemmArgs& a, cudaStream_t s, char* cfg, size_t cfg_len)
   p.norm_cols = a.norm_k != nullptr ? (a.norm_q_heads + a.norm_k_heads) * a.rope_head_dim : p.norm_q_cols;
   p.norm_eps = a.norm_eps;
   p.status = a.status;
+  p.live = a.live, p.block_pos = a.block_pos;
   const int sms = sm_count();
   // Tile width: the widest MMA whose tile count still fills the SMs. A gated
   // tile spends half its MMA width on the up rows; a turned tile must hold

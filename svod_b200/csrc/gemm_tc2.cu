@@ -79,6 +79,8 @@ struct Params2 {
   int rope_width;
   int head_dim;      // 128 (norm and/or rotation), or 64 (rotation only)
   int64_t rope_seq;  // table rows; a tile's 128 rows never wrap around it
+  const int32_t* live;       // nullable: packed rows to compute; tiles past them are not walked
+  const int32_t* block_pos;  // their blocks' positions
 };
 
 using namespace gemm_parts;
@@ -114,7 +116,6 @@ __global__ void __launch_bounds__(32 * (2 + EW), 1)
   const int pair = blockIdx.x >> 1;
   const int pairs = gridDim.x >> 1;
   const int num_kb = (p.k + BK - 1) / BK;
-  const int num_tiles = p.tiles_m * p.tiles_n;
 
   if (threadIdx.x == 0) {
     for (int i = 0; i < S; ++i) {
@@ -137,6 +138,8 @@ __global__ void __launch_bounds__(32 * (2 + EW), 1)
     tmem_relinquish_pair();
   }
   pdl_wait();
+  const int tiles_m = live_tiles(p.live, p.tiles_m, 2 * BM);
+  const int num_tiles = tiles_m * p.tiles_n;
   if (HEADS && threadIdx.x < 256) {
     const T* wsrc = (const T*)(threadIdx.x < 128 ? p.norm_q : p.norm_k);
     head_w[threadIdx.x] = wsrc != nullptr ? Elem<T>::to_f(wsrc[threadIdx.x & 127]) : 1.0f;
@@ -158,7 +161,7 @@ __global__ void __launch_bounds__(32 * (2 + EW), 1)
       bool ok = true;
       for (int t = pair; t < num_tiles && ok; t += pairs) {
         int mt, nt;
-        tile_coords(t, p.tiles_m, p.tiles_n, mt, nt);
+        tile_coords(t, tiles_m, p.tiles_n, mt, nt);
         const int m0 = mt * 2 * BM + (int)rank * BM;
         const int n0 = nt * p.out_bn;
         // this CTA's 128 rows of the W tile: the lower / upper half of a plain
@@ -190,11 +193,16 @@ __global__ void __launch_bounds__(32 * (2 + EW), 1)
             break;
           }
           tab_ph ^= 1;
-          const int row0 = (int)((int64_t)m0 % p.rope_seq);
+          // (in two halves: packed rows are runs of 64 positions)
           mbar_expect_tx(tab_full, (uint32_t)(p.head_dim == 64 ? kTableBytes / 2 : kTableBytes));
-          const int tab_row = p.head_dim == 64 ? row0 / 2 : row0;  // 64-wide heads: two positions per map row
-          tma_load_2d(tables, &tmap_cos, tab_full, 0, tab_row);
-          tma_load_2d(tables + kTableBytes / 2, &tmap_sin, tab_full, 0, tab_row);
+          for (int h = 0; h < 2; ++h) {
+            const int at = m0 + h * kRowBlock;
+            const int row0 = p.live != nullptr ? (at < p.m ? p.block_pos[at / kRowBlock] : 0) : (int)((int64_t)at % p.rope_seq);
+            const int tab_row = p.head_dim == 64 ? row0 / 2 : row0;  // 64-wide heads: two positions per map row
+            uint8_t* dst = tables + h * (p.head_dim == 64 ? kTableBytes / 8 : kTableBytes / 4);
+            tma_load_2d(dst, &tmap_cos, tab_full, 0, tab_row);
+            tma_load_2d(dst + kTableBytes / 2, &tmap_sin, tab_full, 0, tab_row);
+          }
         }
       }
       // Error path: a bounded pause lets copies already in flight land before
@@ -273,7 +281,7 @@ __global__ void __launch_bounds__(32 * (2 + EW), 1)
     int slot = 0;
     for (int t = pair; t < num_tiles; t += pairs) {
       int mt, nt;
-      tile_coords(t, p.tiles_m, p.tiles_n, mt, nt);
+      tile_coords(t, tiles_m, p.tiles_n, mt, nt);
       const int m_at = mt * 2 * BM + (int)rank * BM + quarter * 32;
       const int n_at = nt * BN + group * 64;
       const bool live = m_at < p.m && n_at < p.n;
@@ -366,7 +374,7 @@ __global__ void __launch_bounds__(32 * (2 + EW), 1)
     bool ok = true;
     for (int t = pair; t < num_tiles && ok; t += pairs) {
       int mt, nt;
-      tile_coords(t, p.tiles_m, p.tiles_n, mt, nt);
+      tile_coords(t, tiles_m, p.tiles_n, mt, nt);
       const int n0 = nt * p.out_bn;
       const int cols = p.out_bn / C::kGroups;
       const int c_lo = chalf * cols;
@@ -662,6 +670,7 @@ int run2(const GemmArgs& a, int sms, cudaStream_t s, char* cfg, size_t cfg_len) 
   p.m = a.m, p.n = a.n, p.k = a.k;
   p.gated = a.gated, p.act = a.act, p.has_scale = a.has_scale, p.scale = a.scale;
   p.bias = a.bias, p.residual = a.residual, p.status = a.status;
+  p.live = a.live, p.block_pos = a.block_pos;
   p.out_bn = a.gated ? BN / 2 : BN;
   p.tiles_m = (int)((a.m + 2 * BM - 1) / (2 * BM));
   p.tiles_n = (a.n + p.out_bn - 1) / p.out_bn;
@@ -687,11 +696,11 @@ int run2(const GemmArgs& a, int sms, cudaStream_t s, char* cfg, size_t cfg_len) 
     p.rope_seq = a.rope_seq > 0 ? a.rope_seq : 1;
     if (a.rope_cos != nullptr) {
       // [rope_seq rows, head_dim/2 columns] tables, one 128-position slab per CTA and
-      // tile. 64-wide heads have 64-byte table rows: the map views two positions as
+      // tile, in two boxes. 64-wide heads have 64-byte table rows: the map views two positions as
       // one 128-byte row, so the slab keeps the 128-byte-row swizzle.
       const uint64_t per_row = p.head_dim == 64 ? 2 : 1;
-      if (!make_tmap_2d(&tcos, a.rope_cos, dt, 64, (uint64_t)p.rope_seq / per_row, 64, 64, BM / (uint32_t)per_row)) return -1;
-      if (!make_tmap_2d(&tsin, a.rope_sin, dt, 64, (uint64_t)p.rope_seq / per_row, 64, 64, BM / (uint32_t)per_row)) return -1;
+      if (!make_tmap_2d(&tcos, a.rope_cos, dt, 64, (uint64_t)p.rope_seq / per_row, 64, 64, kRowBlock / (uint32_t)per_row)) return -1;
+      if (!make_tmap_2d(&tsin, a.rope_sin, dt, 64, (uint64_t)p.rope_seq / per_row, 64, 64, kRowBlock / (uint32_t)per_row)) return -1;
     }
   }
   // the attribute belongs to the device's copy of the kernel: once per device
@@ -740,7 +749,7 @@ bool gemm_tc2_covers(const GemmArgs& a) {
     // 128-wide heads (norm and/or rotation), or 64-wide heads with a rotation only
     const bool wide64 = a.rope_head_dim == 64 && a.rope_cos != nullptr && a.norm_q == nullptr && a.norm_k == nullptr;
     if ((a.rope_head_dim != 128 && !wide64) || a.bias != nullptr) return false;
-    if (a.rope_cos != nullptr && (a.rope_seq <= 0 || a.rope_seq % BM != 0)) return false;
+    if (a.rope_cos != nullptr && (a.rope_seq <= 0 || a.rope_seq % (a.live != nullptr ? kRowBlock : BM) != 0)) return false;
   }
   const int out_bn = a.gated ? BN / 2 : BN;
   if (a.n < out_bn || a.m < 2 * BM) return false;

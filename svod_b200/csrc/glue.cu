@@ -22,22 +22,29 @@ template <typename T, typename I>
 __global__ void __launch_bounds__(256)
     embed_kernel(const I* __restrict__ ids, const T* __restrict__ table, const T* __restrict__ pos_table,
                  const T* __restrict__ type_row, int64_t pad_id, T* __restrict__ out, int64_t t_len, int d,
-                 int64_t vocab, int64_t max_pos, int vec16) {
+                 int64_t vocab, int64_t max_pos, int vec16, const int32_t* live, const int32_t* block_seq,
+                 const int32_t* block_pos) {
   __shared__ int red[8];
   __shared__ int64_t tok_id[kTok];
   __shared__ int64_t tok_pos[kTok];
-  const int64_t b = blockIdx.y;
-  const int64_t t0 = (int64_t)blockIdx.x * kTok;
-  const I* row = ids + b * t_len;
   const int tid = threadIdx.x;
   // The first kernel of a stack: it lets the next one up only once all before it is done,
   // so that nothing later ever runs beside what was on the stream before the stack.
   pdl_wait();
   pdl_trigger();
+  int64_t b = blockIdx.y, t0 = (int64_t)blockIdx.x * kTok, o0 = b * t_len + t0;
+  int64_t t_end = t_len;
+  if (live != nullptr) {  // packed rows: the block's first row says which tokens it holds
+    o0 = ((int64_t)blockIdx.y * gridDim.x + blockIdx.x) * kTok;
+    if (o0 >= *reinterpret_cast<const volatile int32_t*>(live)) return;
+    b = block_seq[o0 / kRowBlock], t0 = block_pos[o0 / kRowBlock] + o0 % kRowBlock;
+    t_end = t0 + kTok;  // rows behind the last id are some token too: their values only have to be finite
+  }
+  const I* row = ids + b * t_len;
   int before = 0;
   if (pos_table != nullptr && pad_id >= 0) {
     int cnt = 0;
-    for (int64_t i = tid; i < t0; i += 256) cnt += (int64_t)row[i] != pad_id;
+    for (int64_t i = tid; i < t0 && i < t_len; i += 256) cnt += (int64_t)row[i] != pad_id;
     cnt = (int)warp_sum((float)cnt);  // counts stay below 2^24: exact in f32
     if ((tid & 31) == 0) red[tid >> 5] = cnt;
     __syncthreads();
@@ -47,8 +54,8 @@ __global__ void __launch_bounds__(256)
     int run = before;
     for (int j = 0; j < kTok; ++j) {
       const int64_t t = t0 + j;
-      if (t >= t_len) break;
-      int64_t id = (int64_t)row[t];
+      if (t >= t_end) break;
+      int64_t id = t < t_len ? (int64_t)row[t] : pad_id;
       const bool real = id != pad_id;
       run += real ? 1 : 0;
       tok_pos[j] = pad_id >= 0 ? (real ? run : 0) + pad_id : t;
@@ -59,12 +66,12 @@ __global__ void __launch_bounds__(256)
   const int vec = d / 8;
   for (int j = 0; j < kTok; ++j) {
     const int64_t t = t0 + j;
-    if (t >= t_len) break;
+    if (t >= t_end) break;
     const T* src = table + tok_id[j] * d;
     int64_t p = tok_pos[j];
     p = p < 0 ? 0 : (p >= max_pos ? max_pos - 1 : p);
     const T* psrc = pos_table != nullptr ? pos_table + p * d : nullptr;
-    T* dst = out + (b * t_len + t) * d;
+    T* dst = out + (o0 + j) * d;
     if (!vec16) {
       // an operand off the 16-byte boundary: element by element, same roundings
       for (int c = tid; c < d; c += 256) {
@@ -115,21 +122,28 @@ __global__ void __launch_bounds__(kTok * 32)
     embed_norm_kernel(const I* __restrict__ ids, const T* __restrict__ table, const T* __restrict__ pos_table,
                       const T* __restrict__ type_row, int64_t pad_id, const T* __restrict__ w,
                       const T* __restrict__ b, float eps, int layer, T* __restrict__ out, int64_t t_len,
-                      int64_t vocab, int64_t max_pos) {
+                      int64_t vocab, int64_t max_pos, const int32_t* live, const int32_t* block_seq,
+                      const int32_t* block_pos) {
   constexpr int D = SPANS * 256;
   __shared__ int red[kTok];
   __shared__ int64_t tok_id[kTok];
   __shared__ int64_t tok_pos[kTok];
-  const int64_t bi = blockIdx.y;
-  const int64_t t0 = (int64_t)blockIdx.x * kTok;
-  const I* row = ids + bi * t_len;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   pdl_wait();  // then the trigger: as in embed_kernel
   pdl_trigger();
+  int64_t bi = blockIdx.y, t0 = (int64_t)blockIdx.x * kTok, o0 = bi * t_len + t0;
+  int64_t t_end = t_len;
+  if (live != nullptr) {  // packed rows, as in embed_kernel
+    o0 = ((int64_t)blockIdx.y * gridDim.x + blockIdx.x) * kTok;
+    if (o0 >= *reinterpret_cast<const volatile int32_t*>(live)) return;
+    bi = block_seq[o0 / kRowBlock], t0 = block_pos[o0 / kRowBlock] + o0 % kRowBlock;
+    t_end = t0 + kTok;
+  }
+  const I* row = ids + bi * t_len;
   int before = 0;
   if (pos_table != nullptr && pad_id >= 0) {
     int cnt = 0;
-    for (int64_t i = tid; i < t0; i += kTok * 32) cnt += (int64_t)row[i] != pad_id;
+    for (int64_t i = tid; i < t0 && i < t_len; i += kTok * 32) cnt += (int64_t)row[i] != pad_id;
     cnt = (int)warp_sum((float)cnt);  // counts stay below 2^24: exact in f32
     if (lane == 0) red[warp] = cnt;
     __syncthreads();
@@ -139,8 +153,8 @@ __global__ void __launch_bounds__(kTok * 32)
     int run = before;
     for (int j = 0; j < kTok; ++j) {
       const int64_t t = t0 + j;
-      if (t >= t_len) break;
-      int64_t id = (int64_t)row[t];
+      if (t >= t_end) break;
+      int64_t id = t < t_len ? (int64_t)row[t] : pad_id;
       const bool real = id != pad_id;
       run += real ? 1 : 0;
       tok_pos[j] = pad_id >= 0 ? (real ? run : 0) + pad_id : t;
@@ -149,7 +163,7 @@ __global__ void __launch_bounds__(kTok * 32)
   }
   __syncthreads();
   const int64_t t = t0 + warp;
-  if (t >= t_len) return;
+  if (t >= t_end) return;
   const T* src = table + tok_id[warp] * D;
   int64_t pp = tok_pos[warp];
   pp = pp < 0 ? 0 : (pp >= max_pos ? max_pos - 1 : pp);
@@ -175,7 +189,7 @@ __global__ void __launch_bounds__(kTok * 32)
     }
   }
   const float inv = rows_parts::centre_and_scale<SPANS>(v, eps, layer);
-  T* dst = out + (bi * t_len + t) * D;
+  T* dst = out + (o0 + warp) * D;
 #pragma unroll
   for (int s = 0; s < SPANS; ++s) {
     const int off = s * 256 + lane * 8;
@@ -197,7 +211,8 @@ template <typename T, int SPANS>
 __global__ void __launch_bounds__(256)
     norm_pool_kernel(const T* __restrict__ hidden, const T* __restrict__ w, const T* __restrict__ b, float eps,
                      int layer, const void* __restrict__ aux, int aux_i32, int mode, int slots, int normalize,
-                     float* __restrict__ out, int64_t out_row_stride, int64_t l_len, const PeerPush pp) {
+                     float* __restrict__ out, int64_t out_row_stride, int64_t l_len, const PeerPush pp,
+                     const int32_t* row_start) {
   constexpr int D = SPANS * 256;
   __shared__ float part[8192];  // [warps][D], warps * D <= 8192
   __shared__ float cnts[8];
@@ -205,7 +220,7 @@ __global__ void __launch_bounds__(256)
   pdl_trigger();
   pdl_wait();
   const int64_t bi = mode == 3 ? blockIdx.x / slots : blockIdx.x;
-  const T* h = hidden + bi * l_len * D;
+  const T* h = hidden + (row_start != nullptr ? (int64_t)row_start[bi] : bi * l_len) * D;
   float acc[SPANS][8];
 #pragma unroll
   for (int s = 0; s < SPANS; ++s)
@@ -398,11 +413,14 @@ __global__ void rope_table_kernel(float theta, const int32_t* __restrict__ posit
 
 void launch_embed(const EmbedArgs& a, cudaStream_t s) {
   if (a.batch * a.t == 0) return;
-  dim3 grid((unsigned)((a.t + kTok - 1) / kTok), (unsigned)a.batch);
+  const RowLayout none{};
+  const RowLayout& lay = a.layout != nullptr ? *a.layout : none;
+  dim3 grid((unsigned)(((a.layout != nullptr ? lay.len : a.t) + kTok - 1) / kTok), (unsigned)a.batch);
   const int vec16 = aligned16(a.table) && aligned16(a.pos_table) && aligned16(a.type_row) && aligned16(a.out) ? 1 : 0;
 #define SVODB_EMBED(T, I)                                                                                         \
   launch_pdl(embed_kernel<T, I>, grid, dim3(256), 0, s, 1, (const I*)a.ids, (const T*)a.table,         \
-             (const T*)a.pos_table, (const T*)a.type_row, a.pad_id, (T*)a.out, a.t, a.d, a.vocab, a.max_pos, vec16)
+             (const T*)a.pos_table, (const T*)a.type_row, a.pad_id, (T*)a.out, a.t, a.d, a.vocab, a.max_pos, vec16, lay.live, \
+             lay.block_seq, lay.block_pos)
   if (a.dtype == SVODB_BF16) {
     if (a.ids_i64) SVODB_EMBED(__nv_bfloat16, int64_t);
     else SVODB_EMBED(__nv_bfloat16, int32_t);
@@ -416,12 +434,14 @@ void launch_embed(const EmbedArgs& a, cudaStream_t s) {
 namespace {
 template <typename T, typename I>
 bool embed_norm_dispatch(const EmbedArgs& a, const EmbedNormArgs& n, cudaStream_t s) {
-  dim3 grid((unsigned)((a.t + kTok - 1) / kTok), (unsigned)a.batch);
+  const RowLayout none{};
+  const RowLayout& lay = a.layout != nullptr ? *a.layout : none;
+  dim3 grid((unsigned)(((a.layout != nullptr ? lay.len : a.t) + kTok - 1) / kTok), (unsigned)a.batch);
 #define SVODB_EN(SP)                                                                                                \
   case SP:                                                                                                          \
     launch_pdl(embed_norm_kernel<T, I, SP>, grid, dim3(kTok * 32), 0, s, 1, (const I*)a.ids, (const T*)a.table,      \
                (const T*)a.pos_table, (const T*)a.type_row, a.pad_id, (const T*)n.w, (const T*)n.b, n.eps, n.layer, \
-               (T*)a.out, a.t, a.vocab, a.max_pos);                                                                \
+               (T*)a.out, a.t, a.vocab, a.max_pos, lay.live, lay.block_seq, lay.block_pos);                                                                \
     return true
   switch (a.d / 256) {
     SVODB_EN(1); SVODB_EN(2); SVODB_EN(3); SVODB_EN(4); SVODB_EN(5); SVODB_EN(6); SVODB_EN(7); SVODB_EN(8);
@@ -442,7 +462,7 @@ bool norm_pool_dispatch(const PoolArgs& a, const EmbedNormArgs& n, cudaStream_t 
   case SP:                                                                                                         \
     launch_pdl(norm_pool_kernel<T, SP>, dim3((unsigned)out_rows), dim3(warps * 32), 0, s, 1, (const T*)a.hidden,    \
                (const T*)n.w, (const T*)n.b, n.eps, n.layer, a.aux, a.aux_i32, a.mode, a.slots, a.normalize, a.out, \
-               a.out_row_stride, a.l, pp);                                                                         \
+               a.out_row_stride, a.l, pp, a.row_start);                                                                         \
     return true
   switch (spans) {
     SVODB_NP(1); SVODB_NP(2); SVODB_NP(3); SVODB_NP(4); SVODB_NP(5); SVODB_NP(6); SVODB_NP(7); SVODB_NP(8);

@@ -8,6 +8,34 @@
 
 namespace svodb {
 
+// ---- layout.cu: the rows of a padded batch that a stack really computes -----------
+// A padded batch [B, L] with its rows packed end to end, each cut after its last real
+// token and rounded up to whole blocks of kRowBlock positions. All pointers are device
+// memory that `launch_row_layout` fills; kernels that are given one of them walk the
+// `live` rows instead of all B * L.
+constexpr int kRowBlock = 64;  // = the attention kernel's key block: no key block straddles two rows
+struct RowLayout {
+  int64_t batch, len;        // L rounded up to whole blocks: what the tensors' shapes say
+  const int32_t* live;       // [1] packed rows in all
+  const int32_t* start;      // [B] first packed row of a batch row
+  const int32_t* keys;       // [B] positions up to the last real token
+  const int32_t* rows;       // [B] packed rows of a batch row (whole blocks, one at least)
+  const int32_t* holes;      // [B] nonzero where padding also lies before the last real token
+  const int32_t* block_seq;  // [B * L / kRowBlock] batch row of a packed block
+  const int32_t* block_pos;  // [B * L / kRowBlock] its first position
+};
+struct RowLayoutArgs {
+  const void* mask;        // [B, L] u8 or i32, or null
+  int mask_i32;
+  const int32_t* lengths;  // [B], where there is no mask
+  int64_t batch, len;      // L as the caller has it
+  int32_t* table;          // row_layout_ints(B, L) words, zero before the first launch
+  uint8_t* mask_out;       // [B, L rounded up]: the mask as bytes, zero behind L; nullable
+};
+size_t row_layout_ints(int64_t batch, int64_t len);
+RowLayout row_layout_of(int64_t batch, int64_t len, const int32_t* table);
+void launch_row_layout(const RowLayoutArgs& a, cudaStream_t s);
+
 // ---- rows.cu: LayerNorm / RMSNorm (+ fused residual) ------------------------
 struct NormArgs {
   const void* x;
@@ -21,6 +49,7 @@ struct NormArgs {
   float eps;
   int layer;  // 1 = LayerNorm, 0 = RMSNorm
   int dtype;
+  const int32_t* live;  // nullable: only this many rows are computed
 };
 // Returns 1 when the warp-per-row kernel ran, 0 when the generic one did.
 int launch_norm(const NormArgs& a, cudaStream_t s);
@@ -57,6 +86,7 @@ struct EmbedArgs {
   int d;
   int64_t vocab, max_pos;
   int dtype;
+  const RowLayout* layout;  // nullable: `out` holds the packed rows (ids stay [B, T])
 };
 void launch_embed(const EmbedArgs& a, cudaStream_t s);
 
@@ -84,6 +114,7 @@ struct PoolArgs {
   int64_t batch, l;
   int d;
   int dtype;
+  const int32_t* row_start;  // nullable: `hidden` holds packed rows (fused norm + pool kernel only)
 };
 void launch_pool(const PoolArgs& a, cudaStream_t s);
 
@@ -145,6 +176,7 @@ struct AttnArgs {
   const void* v_app;
   int n_app;
   const int32_t* app_lens;   // [B] or null
+  const RowLayout* layout;   // nullable: q, k, v and o hold packed rows (persistent kernel only)
 };
 // Exact CUDA-core path (any float dtype, any D <= 256, every mask, bias, splits).
 int launch_attention_generic(const AttnArgs& a, cudaStream_t s);
@@ -158,6 +190,8 @@ bool attention_tc_covers(const AttnArgs& a);
 // The persistent form (one CTA per SM over a work queue); same contract.
 int launch_attention_tc_p(const AttnArgs& a, cudaStream_t s, char* cfg, size_t cfg_len);
 bool attention_tc_p_covers(const AttnArgs& a);
+// Whether the persistent kernel can be launched on this stream whatever the item count.
+bool attention_tc_p_ready(cudaStream_t s);
 
 // Few query rows per KV head against many keys (cache slices, row maps, appended
 // rows, bool masks, bias): the keys are read once for all of them; same contract.
@@ -218,6 +252,8 @@ struct GemmArgs {
   int k_splits;
   void* workspace;
   size_t workspace_bytes;
+  const int32_t* live;       // nullable: only this many rows of x are computed (the last tile whole)
+  const int32_t* block_pos;  // with `live`: position of a kRowBlock block's first row, for the rotation tables
   int w_static;  // the caller's word that no launch in flight writes w: its loads need not wait for one
 };
 // `force_bn` codes of the few-tile kernel: kForceSmall + S = a cluster of S CTAs a tile.

@@ -35,12 +35,16 @@ template <typename T, int SPANS, bool RES>
 __global__ void __launch_bounds__(kWarpsPerBlock * 32, rows_blocks(SPANS, RES))
     norm_rows_kernel(const T* __restrict__ x, const T* __restrict__ res, const T* __restrict__ w,
                      const T* __restrict__ b, T* __restrict__ out, T* __restrict__ sum, int64_t rows, float eps,
-                     int layer) {
+                     int layer, const int32_t* live) {
   constexpr int D = SPANS * 256;
   __shared__ uint4 wb[2][SPANS * 32];
   const int lane = threadIdx.x & 31;
   pdl_trigger();
   pdl_wait();
+  if (live != nullptr) {
+    const int64_t n = *reinterpret_cast<const volatile int32_t*>(live);
+    rows = n < rows ? n : rows;
+  }
   const int64_t stride = (int64_t)gridDim.x * kWarpsPerBlock;
   int64_t row = (int64_t)blockIdx.x * kWarpsPerBlock + (threadIdx.x >> 5);
   uint4 xu[SPANS], ru[RES ? SPANS : 1];
@@ -147,7 +151,7 @@ void run_rows(const NormArgs& a, cudaStream_t s) {
   const unsigned blocks = (unsigned)(want < (int64_t)sms * per_sm ? want : (int64_t)sms * per_sm);
   auto* kernel = a.residual != nullptr ? norm_rows_kernel<T, SPANS, true> : norm_rows_kernel<T, SPANS, false>;
   launch_pdl(kernel, dim3(blocks), dim3(kWarpsPerBlock * 32), 0, s, 1, (const T*)a.x, (const T*)a.residual, (const T*)a.w,
-             (const T*)a.b, (T*)a.out, (T*)a.sum, a.rows, a.eps, a.layer);
+             (const T*)a.b, (T*)a.out, (T*)a.sum, a.rows, a.eps, a.layer, a.live);
 }
 
 template <typename T>

@@ -52,6 +52,9 @@ struct svodb_plan {
   void* aux;          // Qwen3: lengths [rows] i32; the others: padding mask [rows, len] bytes
   size_t aux_bytes;
   float* pooled;      // [rows, D]
+  bool packed;        // the stack runs over packed rows (svodb_rows_begin)
+  void* table;        // their layout
+  uint8_t* mask;      // and their key mask
   svodb_graph* graph;
   cudaStream_t stream;
 };
@@ -149,14 +152,18 @@ Acts carve(Bump& b, const svodb_model& m, int64_t B, int64_t L, int reference_op
   return a;
 }
 
+// Positions a row of the activations has room for.
+int64_t padded_len(int64_t len) { return (len + 63) / 64 * 64; }
+int64_t tensor_len(const svodb_plan* p) { return p->packed ? padded_len(p->len) : p->len; }
+
 int forward_qwen3(const svodb_plan* p, const Acts& a, int reference_ops) {
   const svodb_model& m = *p->model;
   const svodb_qwen3_config& c = m.q;
   const int dt = c.dtype;
-  const int64_t B = p->rows, L = p->len, D = c.hidden, H = c.heads, Hkv = c.kv_heads, hd = c.head_dim, F = c.ffn;
+  const int64_t B = p->rows, L = tensor_len(p), D = c.hidden, H = c.heads, Hkv = c.kv_heads, hd = c.head_dim, F = c.ffn;
   const int64_t QKV = (H + 2 * Hkv) * hd;
   void* s = p->stream;
-  svodb_tensor ids = tensor(p->ids, SVODB_I32, {B, L});
+  svodb_tensor ids = tensor(p->ids, SVODB_I32, {B, p->len});
   svodb_tensor table = tensor(m.qw.embed, dt, {c.vocab, D});
   svodb_tensor x = tensor(a.x, dt, {B, L, D});
   svodb_tensor xn = tensor(a.xn, dt, {B, L, D});
@@ -225,10 +232,10 @@ int forward_xlmr(const svodb_plan* p, const Acts& a) {
   const svodb_model& m = *p->model;
   const svodb_xlmr_config& c = m.x;
   const int dt = c.dtype;
-  const int64_t B = p->rows, L = p->len, D = c.hidden, H = c.heads, F = c.ffn;
+  const int64_t B = p->rows, L = tensor_len(p), D = c.hidden, H = c.heads, F = c.ffn;
   void* s = p->stream;
-  svodb_tensor ids = tensor(p->ids, SVODB_I32, {B, L});
-  svodb_tensor mask = tensor(p->aux, SVODB_U8, {B, L});
+  svodb_tensor ids = tensor(p->ids, SVODB_I32, {B, p->len});
+  svodb_tensor mask = tensor(p->packed ? p->mask : p->aux, SVODB_U8, {B, L});
   svodb_tensor word = tensor(m.xw.word, dt, {c.vocab, D});
   svodb_tensor pos = tensor(m.xw.pos, dt, {c.max_positions, D});
   svodb_tensor type = tensor(m.xw.type, dt, {D});
@@ -278,10 +285,10 @@ int forward_modernbert(const svodb_plan* p, const Acts& a) {
   const svodb_model& m = *p->model;
   const svodb_modernbert_config& c = m.m;
   const int dt = c.dtype;
-  const int64_t B = p->rows, L = p->len, D = c.hidden, H = c.heads, F = c.ffn, hd = D / H;
+  const int64_t B = p->rows, L = tensor_len(p), D = c.hidden, H = c.heads, F = c.ffn, hd = D / H;
   void* s = p->stream;
-  svodb_tensor ids = tensor(p->ids, SVODB_I32, {B, L});
-  svodb_tensor mask = tensor(p->aux, SVODB_U8, {B, L});
+  svodb_tensor ids = tensor(p->ids, SVODB_I32, {B, p->len});
+  svodb_tensor mask = tensor(p->packed ? p->mask : p->aux, SVODB_U8, {B, L});
   svodb_tensor table = tensor(m.mw.embed, dt, {c.vocab, D});
   svodb_tensor eln_w = tensor(m.mw.emb_ln_w, dt, {D});
   svodb_tensor x = tensor(a.x, dt, {B, L, D});
@@ -344,12 +351,30 @@ int forward_modernbert(const svodb_plan* p, const Acts& a) {
   return SVODB_OK;
 }
 
-int forward(const svodb_plan* p, const Acts& a, int reference_ops) {
+int forward_rows(const svodb_plan* p, const Acts& a, int reference_ops) {
   switch (p->model->kind) {
     case kQwen3: return forward_qwen3(p, a, reference_ops);
     case kXlmr: return forward_xlmr(p, a);
     default: return forward_modernbert(p, a);
   }
+}
+
+// Over the rows without their trailing padding where that pays and every op has a kernel
+// for it; a plan that meets one that has none runs padded from then on.
+int forward(svodb_plan* p, const Acts& a, int reference_ops) {
+  if (p->packed) {
+    const bool lens = p->model->kind == kQwen3;
+    svodb_tensor aux = lens ? tensor(p->aux, SVODB_I32, {p->rows}) : tensor(p->aux, SVODB_U8, {p->rows, p->len});
+    svodb_tensor mask = tensor(p->mask, SVODB_U8, {p->rows, padded_len(p->len)});
+    int rc = svodb_rows_begin(&aux, p->len, p->table, lens ? nullptr : &mask, p->stream);
+    if (rc == SVODB_OK) {
+      rc = forward_rows(p, a, reference_ops);
+      svodb_rows_end();
+    }
+    if (rc != SVODB_ERR_UNSUPPORTED) return rc;
+    p->packed = false;
+  }
+  return forward_rows(p, a, reference_ops);
 }
 
 int bad(int code, const char* msg) {
@@ -438,7 +463,10 @@ int svodb_model_plan(svodb_model* m, int64_t rows, int64_t len, int32_t referenc
   dry.take((size_t)rows * len * 4);
   dry.take(p->aux_bytes);
   dry.take((size_t)rows * D * 4);
-  carve(dry, *m, rows, len, reference_ops);
+  const size_t table_bytes = svodb_rows_table_bytes(rows, len);
+  dry.take(table_bytes);
+  dry.take((size_t)rows * padded_len(len));
+  carve(dry, *m, rows, padded_len(len), reference_ops);
   p->arena_bytes = dry.at;
   if (cudaStreamCreateWithFlags(&p->stream, cudaStreamNonBlocking) != cudaSuccess) {
     delete p;
@@ -454,22 +482,27 @@ int svodb_model_plan(svodb_model* m, int64_t rows, int64_t len, int32_t referenc
   p->ids = (int32_t*)b.take((size_t)rows * len * 4);
   p->aux = b.take(p->aux_bytes);
   p->pooled = (float*)b.take((size_t)rows * D * 4);
-  Acts a = carve(b, *m, rows, len, reference_ops);
+  p->table = b.take(table_bytes);
+  p->mask = (uint8_t*)b.take((size_t)rows * padded_len(len));
+  p->packed = !reference_ops && svodb_rows_pay(rows, len);
+  Acts a = carve(b, *m, rows, padded_len(len), reference_ops);
+  const int64_t table_len = tensor_len(p);
+  cudaMemsetAsync(p->table, 0, table_bytes, p->stream);
   // inputs until the first run: token 0 everywhere, full-length rows
   cudaMemsetAsync(p->ids, 0, (size_t)rows * len * 4, p->stream);
   if (m->kind == kQwen3) {
     std::vector<int32_t> full((size_t)rows, (int32_t)len);
     cudaMemcpyAsync(p->aux, full.data(), (size_t)rows * 4, cudaMemcpyHostToDevice, p->stream);
     cudaStreamSynchronize(p->stream);  // `full` leaves scope below
-    svodb_tensor cos = tensor(a.cos, m->q.dtype, {len, m->q.head_dim / 2});
-    svodb_tensor sin = tensor(a.sin, m->q.dtype, {len, m->q.head_dim / 2});
+    svodb_tensor cos = tensor(a.cos, m->q.dtype, {table_len, m->q.head_dim / 2});
+    svodb_tensor sin = tensor(a.sin, m->q.dtype, {table_len, m->q.head_dim / 2});
     rc = svodb_rope_table(m->q.rope_theta, nullptr, m->q.head_dim, &cos, &sin, p->stream);
   } else {
     cudaMemsetAsync(p->aux, 1, p->aux_bytes, p->stream);
     if (m->kind == kModernBert) {
       const int32_t hd = m->m.hidden / m->m.heads;
-      svodb_tensor cg = tensor(a.cos, m->m.dtype, {len, hd / 2}), sg = tensor(a.sin, m->m.dtype, {len, hd / 2});
-      svodb_tensor cl = tensor(a.cos2, m->m.dtype, {len, hd / 2}), sl = tensor(a.sin2, m->m.dtype, {len, hd / 2});
+      svodb_tensor cg = tensor(a.cos, m->m.dtype, {table_len, hd / 2}), sg = tensor(a.sin, m->m.dtype, {table_len, hd / 2});
+      svodb_tensor cl = tensor(a.cos2, m->m.dtype, {table_len, hd / 2}), sl = tensor(a.sin2, m->m.dtype, {table_len, hd / 2});
       rc = svodb_rope_table(m->m.global_theta, nullptr, hd, &cg, &sg, p->stream);
       if (rc == SVODB_OK) rc = svodb_rope_table(m->m.local_theta, nullptr, hd, &cl, &sl, p->stream);
     }

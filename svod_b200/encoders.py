@@ -77,6 +77,20 @@ def _randn(gen, shape, dtype, device, sigma=0.02):
     return (torch.randn(shape, generator=gen, device=device, dtype=torch.float32) * sigma).to(dtype)
 
 
+def _over_real_rows(ids: torch.Tensor, aux: torch.Tensor, run):
+    """`run(aux)` over the batch's rows without their trailing padding where that pays
+    and every op of the stack has a kernel for it, over the padded batch otherwise.
+    `aux`: the padding mask `[B, L]` or the lengths `[B]`."""
+    if aux.shape[0] == ids.shape[0] and ops.rows_pay(*ids.shape):
+        try:
+            with ops.PackedRows(aux, ids.shape[1]) as rows:
+                return run(aux if rows.mask is None else rows.mask)
+        except ops.OpsError as e:
+            if e.code != ops.ERR_UNSUPPORTED:
+                raise
+    return run(aux)
+
+
 # --------------------------------------------------------------------------- XLM-R
 class XlmRobertaEncoder:
     def __init__(self, cfg: XlmRobertaConfig, params: Dict):
@@ -131,10 +145,14 @@ class XlmRobertaEncoder:
         return x
 
     def forward(self, ids, mask, out=None, gather=None):
-        h = self.hidden(ids, mask)
         mode = ops.POOL_CLS if self.cfg.pooling == "cls" else ops.POOL_MEAN
-        # post-LN stack: the last layer's norm is the final one; pooling + L2 in one kernel
-        return ops.norm_pool(h, aux=mask if mode == ops.POOL_MEAN else None, mode=mode, out=out, gather=gather)
+
+        def run(mask):
+            h = self.hidden(ids, mask)
+            # post-LN stack: the last layer's norm is the final one; pooling + L2 in one kernel
+            return ops.norm_pool(h, aux=mask if mode == ops.POOL_MEAN else None, mode=mode, out=out, gather=gather)
+
+        return _over_real_rows(ids, mask, run)
 
 
 # --------------------------------------------------------------------------- Qwen3
@@ -199,10 +217,13 @@ class Qwen3Embedder:
         return x
 
     def forward(self, ids, lengths, out=None, gather=None):
-        # final RMSNorm of the pooled (last real) tokens alone, pooling and L2: one kernel
-        x = self.run_layers(ops.embed(ids, self.p["embed"]), w_static=True)
-        return ops.norm_pool(x, self.p["norm_w"], None, self.cfg.rms_norm_eps, layer=False, aux=lengths,
-                             mode=ops.POOL_LAST, out=out, gather=gather)
+        def run(lengths):
+            # final RMSNorm of the pooled (last real) tokens alone, pooling and L2: one kernel
+            x = self.run_layers(ops.embed(ids, self.p["embed"]), w_static=True)
+            return ops.norm_pool(x, self.p["norm_w"], None, self.cfg.rms_norm_eps, layer=False, aux=lengths,
+                                 mode=ops.POOL_LAST, out=out, gather=gather)
+
+        return _over_real_rows(ids, lengths, run) if self.fused_prologue else run(lengths)
 
 
 # --------------------------------------------------------------------------- ModernBERT
@@ -267,11 +288,15 @@ class ModernBertEncoder:
 
     def forward(self, ids, mask, out=None, gather=None):
         c, p = self.cfg, self.p
-        x = self.run_layers(ops.embed_norm(ids, p["embed"], p["emb_ln_w"], None, c.norm_eps), mask, w_static=True)
         mode = ops.POOL_CLS if c.pooling == "cls" else ops.POOL_MEAN
-        # final LayerNorm (of the tokens that are pooled), pooling and L2: one kernel
-        return ops.norm_pool(x, p["final_ln_w"], None, c.norm_eps, aux=mask if mode == ops.POOL_MEAN else None,
-                             mode=mode, out=out, gather=gather)
+
+        def run(mask):
+            x = self.run_layers(ops.embed_norm(ids, p["embed"], p["emb_ln_w"], None, c.norm_eps), mask, w_static=True)
+            # final LayerNorm (of the tokens that are pooled), pooling and L2: one kernel
+            return ops.norm_pool(x, p["final_ln_w"], None, c.norm_eps, aux=mask if mode == ops.POOL_MEAN else None,
+                                 mode=mode, out=out, gather=gather)
+
+        return _over_real_rows(ids, mask, run)
 
 
 # --------------------------------------------------------------------------- plan replay

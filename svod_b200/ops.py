@@ -13,6 +13,7 @@ from __future__ import annotations
 
 import ctypes as C
 import enum
+import threading
 from dataclasses import dataclass
 from typing import Optional, Tuple
 
@@ -504,12 +505,55 @@ def add_rms_norm(x, residual, w, eps: float = 1e-6):
     return s, out
 
 
+# ---------------------------------------------------------------------- packed rows
+class PackedRows:
+    """A padded batch `[B, L]` computed without its trailing padding
+    (`svodb_rows_begin`): while it is entered, this thread's ops take and make tensors
+    `[B, length, ...]`, `length` = L rounded up to 64, that hold the rows end to end.
+    `aux` is the padding mask `[B, L]` or the lengths `[B]`; `mask` is the key mask of
+    the packed rows (None beside lengths). An op that cannot run over them raises
+    `OpsError` with code `ERR_UNSUPPORTED`."""
+
+    def __init__(self, aux: torch.Tensor, length: int):
+        batch = aux.shape[0]
+        self.given = length
+        self.length = -(-length // 64) * 64
+        if aux.dim() == 1 or aux.dtype not in (torch.bool, torch.uint8, torch.int32):
+            aux = aux.to(torch.int32)
+        self.aux = aux.contiguous()
+        self.mask = (torch.empty(batch, self.length, dtype=torch.uint8, device=aux.device) if aux.dim() == 2 else None)
+        self.table = torch.zeros(L.load().svodb_rows_table_bytes(batch, length) // 4, dtype=torch.int32, device=aux.device)
+
+    def __enter__(self) -> "PackedRows":
+        a, m = _desc(self.aux), _desc(self.mask)
+        _check(L.load().svodb_rows_begin(_p(a), self.given, self.table.data_ptr(), _p(m), _stream()))
+        _packed.length = self.length
+        return self
+
+    def __exit__(self, *exc):
+        _packed.length = None
+        L.load().svodb_rows_end()
+
+
+class _PackedState(threading.local):
+    length: Optional[int] = None  # tokens a row of the tensors under `PackedRows`, this thread's
+
+
+_packed = _PackedState()
+ERR_UNSUPPORTED = L.ERR_UNSUPPORTED
+
+
+def rows_pay(batch: int, length: int) -> bool:
+    """Whether a stack runs a batch `[batch, length]` over packed rows."""
+    return bool(L.load().svodb_rows_pay(batch, length))
+
+
 # ----------------------------------------------------------------------------- glue
 def embed(ids, table, pos_table=None, type_row=None, pad_id: int = -1):
     """Token embedding lookup; with `pos_table` and `pad_id >= 0` the XLM-R
     form (model/src/xlm_roberta/embeddings.rs:53-63)."""
     B, T = ids.shape
-    out = torch.empty(B, T, table.shape[1], dtype=table.dtype, device=table.device)
+    out = torch.empty(B, _packed.length or T, table.shape[1], dtype=table.dtype, device=table.device)
     a, b, c, d, e = _desc(ids), _desc(table), _desc(pos_table), _desc(type_row), _desc(out)
     _check(L.load().svodb_embed(_p(a), _p(b), _p(c), _p(d), int(pad_id), _p(e), _stream()))
     return out
@@ -520,7 +564,7 @@ def embed_norm(ids, table, norm_w, norm_b=None, eps: float = 1e-5, pos_table=Non
     """The lookup of `embed` and the embedding norm in one kernel
     (model/src/xlm_roberta/embeddings.rs:53-63: word + position + type, LayerNorm)."""
     B, T = ids.shape
-    out = torch.empty(B, T, table.shape[1], dtype=table.dtype, device=table.device)
+    out = torch.empty(B, _packed.length or T, table.shape[1], dtype=table.dtype, device=table.device)
     a, b, c, d, e = _desc(ids), _desc(table), _desc(pos_table), _desc(type_row), _desc(out)
     w, bb = _desc(norm_w), _desc(norm_b)
     _check(L.load().svodb_embed_norm(_p(a), _p(b), _p(c), _p(d), int(pad_id), _p(w), _p(bb), float(eps), int(layer),

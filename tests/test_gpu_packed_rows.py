@@ -1,0 +1,143 @@
+"""Packed rows: a padded batch computed without its trailing padding gives the pooled rows
+of the padded batch. Sizes sit where the layout can go wrong: rows that end on, before and
+behind a 64-position block, rows of one token and of none, masks with holes, lengths that
+are no multiple of the block, batches through the few-tile, one-CTA and CTA-pair GEMMs."""
+import numpy as np
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+STACKS = ["xlmr", "qwen3", "modernbert"]
+
+
+def _model(kind, hidden=512):
+    from svod_b200 import encoders as E
+    if kind == "xlmr":
+        cfg = E.XlmRobertaConfig(vocab_size=500, hidden_size=hidden, num_hidden_layers=2, num_attention_heads=hidden // 64,
+                                 intermediate_size=2 * hidden, max_position_embeddings=1100)
+        return E.XlmRobertaEncoder.random_init(cfg, seed=3)
+    if kind == "qwen3":
+        cfg = E.Qwen3Config(vocab_size=500, hidden_size=hidden, num_hidden_layers=2, num_attention_heads=hidden // 128,
+                            num_key_value_heads=hidden // 256, intermediate_size=2 * hidden)
+        return E.Qwen3Embedder.random_init(cfg, seed=4)
+    cfg = E.ModernBertConfig(vocab_size=500, hidden_size=hidden, num_hidden_layers=4, num_attention_heads=hidden // 64,
+                             intermediate_size=hidden)
+    return E.ModernBertEncoder.random_init(cfg, seed=5)
+
+
+def _batch(lens, L, kind, holes=False, seed=0):
+    r = np.random.RandomState(seed)
+    ids = torch.full((len(lens), L), 1, dtype=torch.int32)
+    mask = torch.zeros(len(lens), L, dtype=torch.bool)
+    for i, n in enumerate(lens):
+        ids[i, :n] = torch.from_numpy(r.randint(5, 500, n).astype(np.int32))
+        mask[i, :n] = True
+        if holes and n > 8:
+            mask[i, torch.from_numpy(r.choice(n - 1, n // 5, replace=False))] = False
+    aux = torch.tensor(lens, dtype=torch.int32) if kind == "qwen3" else mask
+    return ids.cuda(), aux.cuda()
+
+
+# (row lengths, L): few-tile / one-CTA / CTA-pair projections; L on and off the block
+CASES = [
+    ([130, 1, 64, 65, 63, 128, 200, 7], 200),
+    ([384, 129, 128, 127], 384),
+    ([301, 33, 97, 192, 1, 320], 321),
+    ([1024, 700, 64, 1, 513, 960, 1000, 130], 1024),
+    ([512] * 16, 512),
+]
+
+
+def _close(got, want, kind):
+    # the same roundings of the same values; only the order of a row's key blocks' rescaling may differ
+    tol = {"xlmr": 2e-3, "qwen3": 1.5e-2, "modernbert": 1.2e-2}[kind]
+    got, want = got.double().cpu(), want.double().cpu()
+    assert torch.isfinite(got).all()
+    assert (got - want).norm() <= tol * want.norm()
+    assert ((got - want).norm(dim=1) <= 2 * tol * want.norm(dim=1).clamp_min(1e-30)).all()
+
+
+@pytest.mark.parametrize("kind", STACKS)
+@pytest.mark.parametrize("case", range(len(CASES)))
+def test_matches_the_padded_batch(kind, case, monkeypatch):
+    from svod_b200 import ops
+    lens, L = CASES[case]
+    model = _model(kind)
+    ids, aux = _batch(lens, L, kind, seed=case)
+    assert ops.rows_pay(*ids.shape)
+    got = model.forward(ids, aux)
+    assert ops._packed.length is None
+    ops.device_status()
+    monkeypatch.setattr(ops, "rows_pay", lambda b, n: False)
+    _close(got, model.forward(ids, aux), kind)
+
+
+@pytest.mark.parametrize("kind,pooling", [("xlmr", "cls"), ("xlmr", "mean"), ("modernbert", "mean"), ("modernbert", "cls")])
+@pytest.mark.parametrize("dtype", [torch.bool, torch.int64])
+def test_masks_with_holes_and_empty_rows(kind, pooling, dtype, monkeypatch):
+    from svod_b200 import ops
+    model = _model(kind)
+    model.cfg.pooling = pooling
+    ids, mask = _batch([150, 0, 320, 65, 0], 320, kind, holes=True)
+    mask[3, :] = False
+    mask[3, 40:60] = True  # hidden tokens before and behind
+    mask = mask.to(dtype)
+    got = model.forward(ids, mask)
+    monkeypatch.setattr(ops, "rows_pay", lambda b, n: False)
+    want = model.forward(ids, mask)
+    live = [0, 2, 3] if pooling == "mean" else range(5)  # the mean of no token is zero on both sides
+    _close(got[list(live)], want[list(live)], kind)
+    assert (got[1] == want[1]).all() or pooling == "cls"
+
+
+def test_lengths_outside_the_row(monkeypatch):
+    from svod_b200 import ops
+    model = _model("qwen3")
+    ids, _ = _batch([300] * 4, 300, "qwen3")
+    aux = torch.tensor([-3, 0, 1000, 77], dtype=torch.int32).cuda()
+    got = model.forward(ids, aux)
+    monkeypatch.setattr(ops, "rows_pay", lambda b, n: False)
+    _close(got, model.forward(ids, aux), "qwen3")
+
+
+@pytest.mark.parametrize("kind", STACKS)
+def test_plan_replays_serve_other_lengths(kind, monkeypatch):
+    """One captured plan, batches of other lengths one after the other: nothing of the one
+    before shows, on the Python plan and the native one (whose L is off the block)."""
+    from svod_b200 import encoders as E
+    from svod_b200 import native, ops
+    model = _model(kind)
+    B, L = 6, 300
+    plan = E.Plan(model, B, L, "lengths" if kind == "qwen3" else "mask").capture()
+    run = {"xlmr": native.NativeXlmRoberta, "qwen3": native.NativeQwen3, "modernbert": native.NativeModernBert}[kind](model)
+    for seed, lens in enumerate([[300] * 6, [1, 2, 64, 65, 300, 128], [5] * 6, [256, 257, 255, 1, 300, 64]]):
+        ids, aux = _batch(lens, L, kind, seed=seed)
+        out = torch.empty(B, model.cfg.hidden_size).pin_memory()
+        plan.run(ids.cpu().pin_memory(), aux.cpu().pin_memory(), out)
+        plan.check()
+        nat = run.run(ids.cpu().numpy(), aux.cpu().numpy().astype(run.aux_dtype))
+        with monkeypatch.context() as m:
+            m.setattr(ops, "rows_pay", lambda b, n: False)
+            want = model.forward(ids, aux)
+        _close(out, want, kind)
+        assert (nat == out.numpy()).all()
+
+
+def test_calls_without_a_kernel_fall_back():
+    """A stack whose rows the fused kernels do not take runs padded, and says nothing."""
+    from svod_b200 import encoders as E
+    from svod_b200 import ops
+    cfg = E.ModernBertConfig(vocab_size=500, hidden_size=320, num_hidden_layers=2, num_attention_heads=10,
+                             intermediate_size=320)  # 32-wide heads: the rotation runs outside the store
+    model = E.ModernBertEncoder.random_init(cfg, seed=1)
+    ids, mask = _batch([200, 100, 256, 33], 256, "modernbert")
+    got = model.forward(ids, mask)
+    assert ops._packed.length is None
+    want = ops.pool(model.hidden(ids, mask), mask, ops.POOL_MEAN)
+    _close(got, want, "modernbert")
+    with pytest.raises(ops.OpsError) as e:
+        with ops.PackedRows(mask, 256):
+            ops.heads(torch.empty(4, 256, 960, dtype=torch.bfloat16, device="cuda"), ops.Qkv(10, 10, 32))
+    assert e.value.code == ops.ERR_UNSUPPORTED
+    assert ops._packed.length is None
