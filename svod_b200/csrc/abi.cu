@@ -1231,7 +1231,7 @@ int pool_impl(const char* OP, const svodb_tensor* hidden, const svodb_tensor* no
   a.d = (int)D;
   a.dtype = hidden->dtype;
   if (rows != nullptr) {
-    a.row_start = rows->start;
+    a.row_start = rows->start, a.row_keys = rows->keys;
     if (mode == 2) a.aux = rows->keys;  // the lengths, cut to L as the layout cut them
   }
   if (!fused) {

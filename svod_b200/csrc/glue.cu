@@ -11,6 +11,12 @@ namespace svodb {
 
 namespace {
 
+__device__ __forceinline__ float ld_cluster_f32(uint32_t addr) {
+  float v;
+  asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(addr) : "memory");
+  return v;
+}
+
 // out[b,t,:] = table[ids[b,t]] (+ pos_table[pos_id] + type_row), each add
 // rounded to the element type as the graph's 16-bit adds are
 // (model/src/xlm_roberta/embeddings.rs:53-63). Position ids:
@@ -207,19 +213,30 @@ __global__ void __launch_bounds__(kTok * 32)
 // normalising each, and sums them in f32. The normalised values are rounded to
 // the element type before they are pooled, as the unfused sequence stores them.
 // w == nullptr: the hidden states are pooled as they are. d = SPANS * 256.
+//
+// The masked mean is a serial chain per warp (load a token, two shuffle reductions, add), so
+// it is bound by latency, not by HBM: one block a row took 1730 us for 16 rows of 8192 and
+// 55 us for 8 of 384 (now 188 and 27). A row is therefore walked by a cluster of up to eight blocks, a warp
+// requests its next real token before it reduces the present one, and the first block adds
+// the others' sums up in rank order out of their shared memory (the same bits every run).
 template <typename T, int SPANS>
 __global__ void __launch_bounds__(256)
     norm_pool_kernel(const T* __restrict__ hidden, const T* __restrict__ w, const T* __restrict__ b, float eps,
                      int layer, const void* __restrict__ aux, int aux_i32, int mode, int slots, int normalize,
                      float* __restrict__ out, int64_t out_row_stride, int64_t l_len, const PeerPush pp,
-                     const int32_t* row_start) {
+                     const int32_t* row_start, const int32_t* row_keys) {
   constexpr int D = SPANS * 256;
   __shared__ float part[8192];  // [warps][D], warps * D <= 8192
   __shared__ float cnts[8];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
   pdl_trigger();
   pdl_wait();
-  const int64_t bi = mode == 3 ? blockIdx.x / slots : blockIdx.x;
+  // the cluster of blocks that walks this output row (one block but for the masked mean)
+  uint32_t csz;
+  asm volatile("mov.u32 %0, %%cluster_nctaid.x;" : "=r"(csz));
+  const int share = (int)cluster_ctarank();
+  const int64_t orow = blockIdx.x / csz, orows = gridDim.x / csz;
+  const int64_t bi = mode == 3 ? orow / slots : orow;
   const T* h = hidden + (row_start != nullptr ? (int64_t)row_start[bi] : bi * l_len) * D;
   float acc[SPANS][8];
 #pragma unroll
@@ -229,25 +246,38 @@ __global__ void __launch_bounds__(256)
   float cnt = 0.f;
   int64_t first = 0, last = 1;  // the token range this block walks
   if (mode == 1) {
-    last = l_len;
+    last = row_keys != nullptr ? row_keys[bi] : l_len;
   } else if (mode == 2) {
     first = (int64_t)((const int32_t*)aux)[bi] - 1;
   } else if (mode == 3) {
-    first = (int64_t)((const int32_t*)aux)[blockIdx.x];
+    first = (int64_t)((const int32_t*)aux)[orow];
   }
   if (mode != 1) {
     first = first < 0 ? 0 : (first > l_len - 1 ? l_len - 1 : first);
     last = first + 1;
   }
-  for (int64_t t = first + warp; t < last; t += warps) {
-    if (mode == 1) {
-      const int m = aux_i32 ? ((const int32_t*)aux)[bi * l_len + t] : (int)((const uint8_t*)aux)[bi * l_len + t];
-      if (m == 0) continue;
-      cnt += 1.f;
-    }
+  const int64_t step = (int64_t)warps * csz;
+  for (int64_t t0 = first + share * warps + warp; t0 < last; t0 += 32 * step) {
+   // 32 of the warp's tokens at a time: which of them are real, then those one by one
+   const int64_t tl = t0 + lane * step;
+   bool real = tl < last;
+   if (mode == 1 && real)
+     real = (aux_i32 ? ((const int32_t*)aux)[bi * l_len + tl] : (int)((const uint8_t*)aux)[bi * l_len + tl]) != 0;
+   uint32_t todo = __ballot_sync(0xffffffffu, real);
+   cnt += (float)__popc(todo);
+   uint4 u[SPANS];
+   auto fetch = [&]() {
+     const T* src = h + (t0 + (__ffs((int)todo) - 1) * step) * D + lane * 8;
+#pragma unroll
+     for (int s = 0; s < SPANS; ++s) u[s] = ldg128(src + s * 256);
+   };
+   if (todo != 0u) fetch();
+   while (todo != 0u) {
     float v[SPANS][8];
 #pragma unroll
-    for (int s = 0; s < SPANS; ++s) rows_parts::unpack8<T>(ldg128(h + t * D + s * 256 + lane * 8), v[s]);
+    for (int s = 0; s < SPANS; ++s) rows_parts::unpack8<T>(u[s], v[s]);
+    todo &= todo - 1;
+    if (todo != 0u) fetch();
     if (w != nullptr) {
       const float inv = rows_parts::centre_and_scale<SPANS>(v, eps, layer);
 #pragma unroll
@@ -263,6 +293,7 @@ __global__ void __launch_bounds__(256)
     for (int s = 0; s < SPANS; ++s)
 #pragma unroll
       for (int i = 0; i < 8; ++i) acc[s][i] += v[s][i];
+   }
   }
   if (warps > 1) {
 #pragma unroll
@@ -271,18 +302,44 @@ __global__ void __launch_bounds__(256)
       for (int i = 0; i < 8; ++i) part[warp * D + s * 256 + lane * 8 + i] = acc[s][i];
     if (lane == 0) cnts[warp] = cnt;
     __syncthreads();
-    if (warp != 0) return;
-    cnt = 0.f;
-    for (int k = 0; k < warps; ++k) cnt += cnts[k];
+    if (warp == 0) {
+      cnt = 0.f;
+      for (int k = 0; k < warps; ++k) cnt += cnts[k];
 #pragma unroll
-    for (int s = 0; s < SPANS; ++s)
+      for (int s = 0; s < SPANS; ++s)
 #pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        float t = 0.f;
-        for (int k = 0; k < warps; ++k) t += part[k * D + s * 256 + lane * 8 + i];  // fixed order: reproducible
-        acc[s][i] = t;
-      }
+        for (int i = 0; i < 8; ++i) {
+          float t = 0.f;
+          for (int k = 0; k < warps; ++k) t += part[k * D + s * 256 + lane * 8 + i];  // fixed order: reproducible
+          acc[s][i] = t;
+        }
+    }
   }
+  if (csz > 1) {
+    if (warp == 0 && share != 0) {
+#pragma unroll
+      for (int s = 0; s < SPANS; ++s)
+#pragma unroll
+        for (int i = 0; i < 8; ++i) part[s * 256 + lane * 8 + i] = acc[s][i];
+      if (lane == 0) cnts[0] = cnt;
+    }
+    __syncwarp();
+    cluster_sync_all();
+    if (warp == 0 && share == 0) {
+      for (uint32_t r = 1; r < csz; ++r) {
+        const uint32_t peer = cluster_map(part, r);
+#pragma unroll
+        for (int s = 0; s < SPANS; ++s)
+#pragma unroll
+          for (int i = 0; i < 8; ++i) acc[s][i] += ld_cluster_f32(peer + 4u * (uint32_t)(s * 256 + lane * 8 + i));
+        cnt += ld_cluster_f32(cluster_map(cnts, r));
+      }
+    }
+    __syncwarp();
+    cluster_sync_all();  // no block leaves before its sums have been read
+    if (share != 0) return;
+  }
+  if (warp != 0) return;
   if (mode == 1) {
     const float invc = 1.0f / fmaxf(cnt, 1e-9f);
 #pragma unroll
@@ -302,7 +359,7 @@ __global__ void __launch_bounds__(256)
 #pragma unroll
       for (int i = 0; i < 8; ++i) acc[s][i] *= inv;
   }
-  float* dst = out + (int64_t)blockIdx.x * out_row_stride;
+  float* dst = out + orow * out_row_stride;
 #pragma unroll
   for (int s = 0; s < SPANS; ++s) {
     float4* d4 = reinterpret_cast<float4*>(dst + s * 256 + lane * 8);
@@ -313,7 +370,7 @@ __global__ void __launch_bounds__(256)
   // stores over NVLink) — the send half of the all-gather, in the kernel that made the row.
   if (pp.world > 1) {
     const uint32_t step = *reinterpret_cast<volatile uint32_t*>(pp.local);
-    const size_t slot = (((size_t)(step & 1u) * pp.world + pp.rank) * gridDim.x + blockIdx.x) * D;
+    const size_t slot = (((size_t)(step & 1u) * pp.world + pp.rank) * orows + orow) * D;
     for (int p = 0; p < pp.world; ++p) {
       if (p == pp.rank) continue;
       float* pd = pp.stage[p] + slot;
@@ -326,7 +383,7 @@ __global__ void __launch_bounds__(256)
     }
     __threadfence_system();
     __syncwarp();
-    if (lane == 0 && atomicAdd(&pp.local[1], 1u) == gridDim.x - 1) {
+    if (lane == 0 && atomicAdd(&pp.local[1], 1u) == (uint32_t)(orows - 1)) {
       __threadfence_system();
       for (int p = 0; p < pp.world; ++p)
         if (p != pp.rank) *reinterpret_cast<volatile uint32_t*>(pp.flags[p] + pp.rank) = step + 1u;
@@ -457,12 +514,16 @@ bool norm_pool_dispatch(const PoolArgs& a, const EmbedNormArgs& n, cudaStream_t 
   const int spans = a.d / 256;
   int warps = 1;
   if (a.mode == 1) warps = spans <= 4 ? 8 : (spans <= 8 ? 4 : 1);
+  // Blocks a row: while a warp keeps four tokens or more, and the rows leave SMs idle.
+  int blocks = 1;
+  if (a.mode == 1 && warps > 1)
+    while (blocks < 8 && a.l >= (int64_t)blocks * 2 * warps * 4 && out_rows * blocks < 296) blocks *= 2;
   const PeerPush pp = a.push != nullptr ? *a.push : PeerPush{};
 #define SVODB_NP(SP)                                                                                               \
   case SP:                                                                                                         \
-    launch_pdl(norm_pool_kernel<T, SP>, dim3((unsigned)out_rows), dim3(warps * 32), 0, s, 1, (const T*)a.hidden,    \
+    launch_pdl(norm_pool_kernel<T, SP>, dim3((unsigned)(out_rows * blocks)), dim3(warps * 32), 0, s, blocks, (const T*)a.hidden,    \
                (const T*)n.w, (const T*)n.b, n.eps, n.layer, a.aux, a.aux_i32, a.mode, a.slots, a.normalize, a.out, \
-               a.out_row_stride, a.l, pp, a.row_start);                                                                         \
+               a.out_row_stride, a.l, pp, a.row_start, a.row_keys);                                                                         \
     return true
   switch (spans) {
     SVODB_NP(1); SVODB_NP(2); SVODB_NP(3); SVODB_NP(4); SVODB_NP(5); SVODB_NP(6); SVODB_NP(7); SVODB_NP(8);

@@ -115,6 +115,7 @@ struct PoolArgs {
   int d;
   int dtype;
   const int32_t* row_start;  // nullable: `hidden` holds packed rows (fused norm + pool kernel only)
+  const int32_t* row_keys;   // with them: positions up to a row's last real token
 };
 void launch_pool(const PoolArgs& a, cudaStream_t s);
 
