@@ -131,10 +131,21 @@ __global__ void __launch_bounds__(kThreadsFa, 1)
     const int tid = threadIdx.x - 64;
     int first_zero = 0x7fffffff, last_set = 0;
     const int words = (int)((p.tk + 31) / 32);
+    const bool vec = !p.key_mask_i32 && (p.tk & 31) == 0 && (reinterpret_cast<uintptr_t>(p.key_mask) & 15) == 0;
     for (int wd = tid; wd < words; wd += 64) {
       uint32_t bits = 0;
       const int64_t base = (int64_t)wd * 32;
-      for (int e = 0; e < 32; ++e) {
+      if (vec) {
+        // 32 byte flags by two 16-byte loads; four 0/1 bytes times 0x10204080 have their bits on top
+        const uint4* src = reinterpret_cast<const uint4*>((const uint8_t*)p.key_mask + b * p.tk + base);
+        const uint4 u = ldg128(src), v = ldg128(src + 1);
+        const uint32_t q[8] = {u.x, u.y, u.z, u.w, v.x, v.y, v.z, v.w};
+#pragma unroll
+        for (int e = 0; e < 8; ++e) bits |= (((__vcmpne4(q[e], 0u) & 0x01010101u) * 0x10204080u) >> 28) << (4 * e);
+        if (bits != 0u) last_set = (int)base + 32 - __clz((int)bits);
+        if (bits != 0xffffffffu && first_zero == 0x7fffffff) first_zero = (int)base + __ffs((int)~bits) - 1;
+      }
+      for (int e = vec ? 32 : 0; e < 32; ++e) {
         const int64_t j = base + e;
         if (j < p.tk) {
           const int64_t at = b * p.tk + j;
