@@ -149,8 +149,10 @@ __global__ void __launch_bounds__(kThreads, 2)
   const int kb0 = rank * per < num_kb ? rank * per : num_kb;
   const int nkb = num_kb - kb0 < per ? num_kb - kb0 : per;
 
-  auto load_w = [&](int i) {
-    const int s = i % p.stages;
+  // Stage numbers and phases run along as counters: a division by the stage count per k-block
+  // costs the one thread that loads (or issues) 500 cycles, more than the block's MMAs
+  // (128 x 1024 x 4096 over 8 CTAs a tile 8.7 -> 7.7 us).
+  auto load_w = [&](int i, int s) {
     uint8_t* dst = smem + (size_t)s * stage_bytes + a_bytes;
     mbar_expect_tx(&full[s], (uint32_t)stage_bytes);
     const int x = (kb0 + i) * BK;
@@ -161,8 +163,7 @@ __global__ void __launch_bounds__(kThreads, 2)
       tma_load_2d(dst, &tmap_w, &full[s], x, n0);
     }
   };
-  auto load_a = [&](int i) {
-    const int s = i % p.stages;
+  auto load_a = [&](int i, int s) {
     tma_load_2d(smem + (size_t)s * stage_bytes, &tmap_a, &full[s], (kb0 + i) * BK, m0);
   };
   const int ahead = nkb < p.stages ? nkb : p.stages;
@@ -178,7 +179,7 @@ __global__ void __launch_bounds__(kThreads, 2)
     mbar_fence_init();
     if (S > 1 && mine > 0) mbar_expect_tx(red_full, (uint32_t)((S - 1) * mine * kPitch * 4));
     if (p.w_static)
-      for (int i = 0; i < ahead; ++i) load_w(i);
+      for (int i = 0; i < ahead; ++i) load_w(i, i);
   }
   if (warp == 1) {
     tmem_alloc(tmem_slot, BN);
@@ -195,13 +196,16 @@ __global__ void __launch_bounds__(kThreads, 2)
     if (lane == 0) {
       pdl_wait();
       bool ok = true;
-      for (int i = 0; i < nkb && ok; ++i) {
-        if (i >= p.stages && !mbar_wait(&empty[i % p.stages], ((i / p.stages) - 1) & 1, p.status)) {
+      int s = 0;
+      uint32_t ph = 1;  // the parity of a stage nobody has used yet
+      for (int i = 0; i < nkb; ++i) {
+        if (i >= p.stages && !mbar_wait(&empty[s], ph, p.status)) {
           ok = false;
           break;
         }
-        if (!p.w_static || i >= ahead) load_w(i);
-        load_a(i);
+        if (!p.w_static || i >= ahead) load_w(i, s);
+        load_a(i, s);
+        if (++s == p.stages) s = 0, ph ^= 1;
       }
       if (!ok)
         for (int i = 0; i < 64; ++i) __nanosleep(1000);  // copies in flight land before the CTA's memory goes
@@ -212,9 +216,10 @@ __global__ void __launch_bounds__(kThreads, 2)
     const bool leader = elect_one();
     const uint64_t desc0 = umma_desc_sw128(smem_u32(smem), 16, 1024);
     bool ok = true;
+    int s = 0;
+    uint32_t ph = 0;
     for (int i = 0; i < nkb; ++i) {
-      const int s = i % p.stages;
-      if (!mbar_wait(&full[s], (i / p.stages) & 1, p.status)) {
+      if (!mbar_wait(&full[s], ph, p.status)) {
         ok = false;
         break;
       }
@@ -225,7 +230,7 @@ __global__ void __launch_bounds__(kThreads, 2)
       for (int k4 = 0; k4 < BK / 16; ++k4)
         if (leader) umma_ss(tmem, ad + (uint64_t)(k4 * 2), wd + (uint64_t)(k4 * 2), idesc, (i | k4) != 0 ? 1u : 0u);
       if (leader) tc_commit(&empty[s]);
-      __syncwarp();
+      if (++s == p.stages) s = 0, ph ^= 1;
     }
     if (ok && leader) tc_commit(acc_full);
     __syncwarp();
@@ -452,32 +457,51 @@ int run_s(const GemmArgs& a, int splits, cudaStream_t s, char* cfg, size_t cfg_l
 }  // namespace
 
 // Measured against the persistent kernels, us a launch in a graph, each launch with weights of
-// its own (M x N x K, best of both, this kernel | the other):
-//   32 x 1024 x 1024     4.3 | 8.2       128 x 1024 x 1024    5.8 | 8.6      256 x 1024 x 1024   7.0 | 8.7
-//   32 x 1024 x 4096     7.3 | 16.6      128 x 1024 x 4096    9.3 | 17.3     256 x 1024 x 4096  13.0 | 17.5
-//   32 x 3072 x 1024     5.6 | 7.1       128 x 3072 x 1024    8.1 | 7.9      512 x 1024 x 4096  21.2 | 17.5
-//   32 x 4096 x 1024 with the attention prologue  6.4 | 14.2;  128 rows  10.4 | 15.6;  256 rows  13.3 | 15.7
-// A tile of at most 64 rows is cheap to send, so it pays up to 100 tiles (two CTAs an SM);
-// fuller tiles up to 48, or 75 where the other kernel needs whole 128-wide heads twice in a
-// 256-column tile. CTAs a tile: as many as the chip holds, 8 at most, two k-blocks each.
+// its own (M x N x K, this kernel | the better of the others):
+//   32 x 1024 x 1024     3.9 | 8.2       128 x 1024 x 1024    5.8 | 8.5      512 x 1024 x 1024   7.1 | 8.9
+//   32 x 1024 x 4096     5.6 | 17.3      128 x 1024 x 4096    7.7 | 18.0     512 x 1024 x 4096  12.3 | 18.3
+//   32 x 3072 x 1024     5.2 | 8.0       128 x 3072 x 1024    7.0 | 8.7      256 x 3072 x 1024   8.3 | 8.8
+//   32 x 4096 x 1024 with the attention prologue  6.1 | 14.3;  128 rows  10.0 | 16.1;  256 rows  12.3 | 16.1
+// Where the lines lie:
+//   * up to 64 rows a tile is cheap to send, so it pays up to 100 tiles, two CTAs an SM; slices
+//     of four k-blocks (64 x 1152 gated x 768: 4.9 us in three CTAs a tile, 5.4 in five);
+//   * a slice of at most nine blocks (three rounds of three stages) leaves room for two CTAs an
+//     SM: two CTAs a tile up to 110 tiles (384 x 2304 x 768 rotated 8.2 | 9.1 us, 384 x 3072 x
+//     1024 with 144 tiles 9.3 | 8.8);
+//   * a longer one takes the whole SM, where clusters of three do not all find a place at once
+//     (48 tiles of K 4096: 19 us, in pairs 12.9), and 128-column tiles halve what is read of x:
+//     512 x 1024 x 4096 12.3 us in four CTAs a tile against 13.5 in two of 64 columns, 1024 rows
+//     16.6 | 18.4; at K 2048 the narrow pairs are ahead (512 x 1024 x 2048 9.8, 10.3 | 11.6);
+//   * whole 128-wide heads up to 75 tiles (384 rows x 4096: 17.8 | 16.1).
 int gemm_small_splits(const GemmArgs& a) {
   if (!gemm_tc_covers(a)) return 0;
   const bool per_head = a.rope_cos != nullptr || a.norm_q != nullptr || a.norm_k != nullptr;
+  if (a.force_bn > kForceSmall && (a.force_bn & 15) <= 8) return a.force_bn - kForceSmall;
   const int bn = per_head ? a.rope_head_dim : 64;
   const int out_bn = a.gated ? bn / 2 : bn;
   const int64_t tiles = ((a.m + BM - 1) / BM) * ((a.n + out_bn - 1) / out_bn);
-  if (a.force_bn > kForceSmall && a.force_bn <= kForceSmall + 8) return a.force_bn - kForceSmall;
-  if (tiles > (a.m <= 64 ? 100 : bn == 128 ? 75 : 48)) return 0;
-  const int64_t room = a.m <= 64 ? 200 : sm_count_s();
   const int kb = (a.k + BK - 1) / BK;
-  int s = (int)(room / tiles < 8 ? room / tiles : 8);
-  if (s > kb / 2) s = kb / 2;
-  return s < 1 ? 1 : s;
+  auto fill = [&](int64_t room, int most) {  // CTAs a tile: as many as the chip holds, eight at most
+    int64_t s = room / tiles < 8 ? room / tiles : 8;
+    if (s > most) s = most;
+    return s < 1 ? 1 : (int)s;
+  };
+  if (a.m <= 64) return tiles <= 100 ? fill(200, bn == 128 ? kb / 2 : (kb + 3) / 4) : 0;
+  if (bn == 128) return tiles <= 75 ? fill(sm_count_s(), kb / 2) : 0;
+  if (kb <= 18) {
+    if (tiles <= 48) return fill(sm_count_s(), kb / 2);
+    return tiles <= 110 && a.m < 1024 ? 2 : 0;
+  }
+  if (tiles <= 18) return 8;
+  if (tiles <= 36) return 4;
+  if (tiles <= 64) return kb >= 40 && !per_head ? kSmallWide + 4 : 2;
+  return tiles <= 128 && kb >= 64 && !per_head ? kSmallWide + 2 : 0;
 }
 
 int launch_gemm_small(const GemmArgs& a, int splits, cudaStream_t s, char* cfg, size_t cfg_len) {
   const bool per_head = a.rope_cos != nullptr || a.norm_q != nullptr || a.norm_k != nullptr;
-  const bool wide = per_head && a.rope_head_dim == 128;
+  const bool wide = per_head ? a.rope_head_dim == 128 : (splits & kSmallWide) != 0;
+  splits &= kSmallWide - 1;
   if (a.dtype == SVODB_BF16)
     return wide ? run_s<__nv_bfloat16, 128>(a, splits, s, cfg, cfg_len) : run_s<__nv_bfloat16, 64>(a, splits, s, cfg, cfg_len);
   return wide ? run_s<__half, 128>(a, splits, s, cfg, cfg_len) : run_s<__half, 64>(a, splits, s, cfg, cfg_len);

@@ -257,9 +257,12 @@ struct GemmArgs {
   const int32_t* block_pos;  // with `live`: position of a kRowBlock block's first row, for the rotation tables
   int w_static;  // the caller's word that no launch in flight writes w: its loads need not wait for one
 };
-// `force_bn` codes of the few-tile kernel: kForceSmall + S = a cluster of S CTAs a tile.
+// `force_bn` codes of the few-tile kernel: kForceSmall + S = a cluster of S CTAs a tile of 64
+// accumulator columns, + kSmallWide = of 128 (a per-head store's tile is its head).
 constexpr int kForceSmall = 1024;
-// The few-tile kernel: CTAs per tile it would run the call with, 0 where another kernel is the better one.
+constexpr int kSmallWide = 16;
+// The few-tile kernel: CTAs per tile it would run the call with (+ kSmallWide), 0 where another
+// kernel is the better one.
 int gemm_small_splits(const GemmArgs& a);
 int launch_gemm_small(const GemmArgs& a, int splits, cudaStream_t s, char* cfg, size_t cfg_len);
 // Workspace bytes of a split-K GEMM: [tiles][2] counters, then [tiles][splits][2][128][256] f32.

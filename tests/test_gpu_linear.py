@@ -421,3 +421,32 @@ def test_device_gelu_is_within_5e_6_of_erf_gelu_on_a_dense_grid():
     assert "kernel gemm" in ops.chosen()
     want = O.round_to(O.BF16, O.gelu_as(xb))
     assert np.max(np.abs(gb - want) / np.maximum(np.abs(want), 1e-2)) < 2.0 ** -7
+
+
+@pytest.mark.parametrize("m,n,k,gated,tile", [
+    (64, 1152, 768, True, "bn:64,"),      # four k-blocks a slice, two CTAs an SM
+    (65, 3072, 1024, False, "bn:64,"),    # first row of a second half tile
+    (384, 2304, 768, False, "cluster:2"),  # 108 tiles, a short k loop in pairs
+    (100, 1024, 4096, False, "cluster:8"),
+    (129, 1024, 4096, True, "bn:128,"),   # gated tiles of 2 x 64 columns, two tile rows
+    (509, 1000, 4096, False, "bn:128,"),  # the last 128-column tile is 104 wide, the last row tile 125 high
+    (1000, 968, 4104, True, ""),          # past the few-tile kernel, K off the 64-column block
+    (900, 1024, 4096, False, "bn:128,"),  # a long slice in two CTAs a tile
+    (300, 768, 2048, False, "cluster:4"),
+    (512, 1024, 2048, False, "cluster:2"),
+])
+def test_few_tile_calls_match_f64(m, n, k, gated, tile):
+    g = torch.Generator(device="cuda").manual_seed(m + n)
+    dt = torch.bfloat16
+    r = lambda s, *shape: (torch.randn(*shape, generator=g, device="cuda") * s).to(dt)
+    k = k // 16 * 16
+    x, w, b = r(1.0, m, k), r(0.02, 2 * n if gated else n, k), r(0.5, 2 * n if gated else n)
+    res = r(1.0, m, n)
+    opts = ops.Linear(bias=b, act=ops.Act.SILU if gated else ops.Act.NONE, gated=gated, residual=res)
+    got = ops.linear(x, w, opts)
+    assert tile in ops.chosen(), ops.chosen()
+    z = x.double() @ w.double().T + b.double()
+    want = (z[:, :n] * torch.sigmoid(z[:, :n]) * z[:, n:] if gated else z) + res.double()
+    # one rounding to bf16 (2^-9 of the value at most), f32 sums below that
+    assert ((got.double() - want).abs() <= 2.0 ** -8 * want.abs() + 1e-3).all()
+    assert torch.equal(got, ops.linear(x, w, opts))  # partials are summed in a fixed order
