@@ -590,6 +590,30 @@ int sm_count_dec() {
   return sms;
 }
 
+int64_t dec_blocks(const AttnArgs& a) { return (a.tk + kKeys - 1) / kKeys + (a.n_app + kKeys - 1) / kKeys; }
+
+// Shares per (lane, KV head): as many as bring the grid to the CTAs the chip holds at
+// once; a second wave of short shares costs its fixed 5 us again (B10 x 4 heads x 1750
+// keys: 12.7 us with 4 shares, 19.9 with 8). Shares that stay at 32 blocks or more hide
+// that, and lanes of unequal length then balance better (B16 x 16 heads x 16384 keys,
+// lengths from 5000: 68 us with 4 shares, 110 with 1). 16 is the largest cluster.
+// A cluster has to find its CTAs' places within one GPC, and large ones do not all find
+// them: sixteen CTAs are worth it up to six clusters per CTA an SM holds (24 pairs x 61
+// blocks, three an SM: 21.8 us in sixteen, 14.1 in eight; 16 pairs x 126 blocks 16.6 against
+// 21.1), eight with one CTA an SM up to twelve (16 pairs x 32 blocks x 32 rows: 41.8 us in
+// eight, 31.2 in four; 8 pairs 22.7 against 31.2).
+int dec_cluster(int64_t pairs, int64_t blocks, int per_sm) {
+  const int64_t room = (int64_t)sm_count_dec() * per_sm;
+  int csize = 1;
+  while (csize < 16 && csize * 2 <= blocks &&
+         (pairs * csize * 2 <= room || (pairs * csize < 4 * room && blocks >= 32 * csize * 2))) {
+    if (csize == 8 && pairs > 6 * per_sm) break;
+    if (csize == 4 && per_sm == 1 && pairs > 12) break;
+    csize *= 2;
+  }
+  return csize;
+}
+
 template <typename T, int D, int NQ>
 int run_dec(const AttnArgs& a, cudaStream_t s, char* cfg, size_t cfg_len) {
   using C = DecCfg<D, NQ>;
@@ -636,18 +660,8 @@ int run_dec(const AttnArgs& a, cudaStream_t s, char* cfg, size_t cfg_len) {
   p.n_app = a.n_app, p.app_lens = a.app_lens;
   p.bias = a.bias, p.bias_per_batch = a.bias_per_batch;
   p.lse = a.lse, p.status = a.status;
-  // Shares per (lane, KV head): as many as bring the grid to the CTAs the chip holds at
-  // once; a second wave of short shares costs its fixed 5 us again (B10 x 4 heads x 1750
-  // keys: 12.7 us with 4 shares, 19.9 with 8). Shares that stay at 32 blocks or more hide
-  // that, and lanes of unequal length then balance better (B16 x 16 heads x 16384 keys,
-  // lengths from 5000: 68 us with 4 shares, 110 with 1). 16 is the largest cluster.
   const int64_t pairs = a.batch * a.kv_heads;
-  const int64_t blocks = (a.tk + kKeys - 1) / kKeys + (a.n_app + kKeys - 1) / kKeys;
-  const int64_t room = (int64_t)sm_count_dec() * C::kPerSm;
-  int csize = 1;
-  while (csize < 16 && csize * 2 <= blocks &&
-         (pairs * csize * 2 <= room || (pairs * csize < 4 * room && blocks >= 32 * csize * 2)))
-    csize *= 2;
+  const int csize = dec_cluster(pairs, dec_blocks(a), C::kPerSm);
   if (launch_pdl(attention_decode_kernel<T, D, NQ>, dim3((unsigned)(pairs * csize)), dim3(kThreadsDec), C::kSmem, s,
                  (unsigned)csize, tk, tv, tka, tva, p) != cudaSuccess)
     return -1;
@@ -666,12 +680,15 @@ int run_dec_rows(const AttnArgs& a, cudaStream_t s, char* cfg, size_t cfg_len) {
 
 }  // namespace
 
-// Up to 16 query rows per KV head, no mask that depends on the query row. From 17 rows on
-// the 256-row tile of the other kernels costs no more per key (B32 x T16 x 4 heads a KV
-// head, 4000 keys: 234 us there, 288 here), but they take no appended rows: those come
-// here up to 64 rows instead of the exact kernel (B5 x T16 x 4 x 8, 1111 + 3 keys: 48 us
-// against 1.1 ms). Key splits the caller asked for stay with the kernel that leaves them
-// in the caller's workspace, appended rows excepted.
+// No mask that depends on the query row, and up to 16 query rows per KV head: always.
+// With 17 to 64 rows a block of 128 keys costs a CTA here 2.6 us (up to 32 rows) or 4.5 us,
+// shared by its cluster; the 256-row tile kernels take 1.55 us for it per head (per pair of
+// heads once there are more pairs than SMs), whatever the rows, and never share a head's
+// keys: the cheaper of the two takes the call (B1 x T4 x 8 heads a KV head, 16000 keys: 34 us
+// here, 203 there; B2 x T16 x 4 heads, 20510 keys: 180 | 249; B32 x T16 x 4 heads, 4000
+// keys: 435 | 320). Appended rows of up to 64 rows always come here, not to the exact
+// kernel (B5 x T16 x 4 x 8, 1111 + 3 keys: 48 us against 1.1 ms). Key splits the caller asked
+// for stay with the kernel that leaves them in the caller's workspace, appended rows excepted.
 bool attention_decode_covers(const AttnArgs& a) {
   AttnArgs plain = a;
   plain.splits = 1;
@@ -680,10 +697,20 @@ bool attention_decode_covers(const AttnArgs& a) {
   if (!attention_tc_covers(plain)) return false;
   if (a.causal || a.has_window || a.has_chunk || a.seg_start != nullptr) return false;
   if (a.splits > 1 && a.n_app == 0) return false;
-  if (a.t > 64 || a.t * (a.heads / a.kv_heads) > (a.n_app > 0 ? 64 : 16)) return false;
-  if (a.batch * a.kv_heads > (1 << 26)) return false;
-  if (a.n_app > 0 && (!aligned16(a.k_app) || !aligned16(a.v_app))) return false;
-  return true;
+  const int64_t group = a.heads / a.kv_heads, rows = a.t * group;
+  if (a.t > 64 || rows > 64) return false;
+  const int64_t pairs = a.batch * a.kv_heads;
+  if (pairs > (1 << 26)) return false;
+  if (a.n_app > 0) return aligned16(a.k_app) && aligned16(a.v_app);
+  if (rows <= 16) return true;
+  const int64_t sms = sm_count_dec(), blocks = dec_blocks(a);
+  const int64_t c = dec_cluster(pairs, blocks, 1);
+  const int64_t head_pairs = group % 2 == 0 ? a.batch * a.heads / 2 : 0;
+  const int64_t items = head_pairs > sms ? head_pairs : a.batch * a.heads;
+  auto up = [](int64_t x, int64_t y) { return (double)((x + y - 1) / y); };
+  const double here = 8.0 + (rows <= 32 ? 2.6 : 4.5) * up(blocks, c) * up(pairs * c, sms);
+  const double there = 4.0 + 1.55 * (double)blocks * up(items, sms);
+  return here < 0.9 * there;
 }
 
 int launch_attention_decode(const AttnArgs& a, cudaStream_t s, char* cfg, size_t cfg_len) {

@@ -633,6 +633,8 @@ DECODE_CASES = [
     (2, 8, 300, 16, 2, 128, 130, "lens"),    # 64 rows, appended rows in two blocks
     (200, 1, 60, 4, 4, 64, 3, "lens"),       # more (lane, head) pairs than the chip holds
     (2, 3, 513, 4, 4, 128, 0, "bool"),       # a bool mask with holes
+    (2, 4, 2050, 16, 2, 128, 0, "lens"),     # 32 rows, no appended row: shared keys beat a tile per head
+    (1, 16, 4100, 8, 2, 64, 0, "bool"),      # 64 rows, four clusters of sixteen
 ]
 
 
