@@ -209,8 +209,8 @@ size_t svodb_attention_workspace_bytes(int64_t batch, int64_t t, int64_t heads, 
  * q [B,T,H,D], k,v [B,Tk,Hkv,D] sequence-major -> o [B,T,H,D].
  * Calls with more work items (256 query rows x head x batch lane) than the
  * device has SMs run a persistent kernel that hands the items out through a
- * counter inside the library, one counter per (device, stream) pair, zeroed on
- * the stream before each launch (a memset node under capture). Launches on one
+ * counter inside the library, one counter per (device, stream) pair, which each
+ * launch leaves at zero for the next. Launches on one
  * stream follow one another, so they may share it; a captured graph keeps the
  * counter of the stream it was captured on, so two graphs captured on the SAME
  * stream must not be replayed at the same time on different streams. Config key
