@@ -557,9 +557,10 @@ __global__ void __launch_bounds__(kThreadsDec, (DecCfg<D, NQ>::kPerSm))
       float l = 0.f, acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
       for (uint32_t r = 0; r < csize; ++r) {
         const float mr = ld_cluster_f32(peer(ml_addr + c * 4, r));
-        if (mr == -INFINITY) continue;  // an empty share
-        const float w = ex2_approx(mr - m);
-        l = fmaf(w, ld_cluster_f32(peer(ml_addr + (NQ + c) * 4, r)), l);
+        const float lr = ld_cluster_f32(peer(ml_addr + (NQ + c) * 4, r));
+        if (lr == 0.f) continue;  // the share saw no key (its sum says so: NaN scores leave the maximum at -inf too)
+        const float w = mr == -INFINITY ? 1.f : ex2_approx(mr - m);
+        l = fmaf(w, lr, l);
         const uint32_t src = peer(op_addr + (c * D + d0) * 4, r);
         const float4 x = ld_cluster_f32x4(src), y = ld_cluster_f32x4(src + 16);
         acc[0] = fmaf(w, x.x, acc[0]), acc[1] = fmaf(w, x.y, acc[1]), acc[2] = fmaf(w, x.z, acc[2]);

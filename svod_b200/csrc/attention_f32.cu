@@ -264,9 +264,10 @@ __global__ void __launch_bounds__(kThreadsF, D == 64 ? 2 : 1) attention_f32_kern
       float sum = 0.f;
       for (int r = 0; r < shares; ++r) {
         const float mr = ld_peer(ml + row, r);
-        if (mr == -INFINITY) continue;  // an empty share
-        const float w = exp2f(mr - mx);
-        sum = fmaf(w, ld_peer(ml + kTile + row, r), sum);
+        const float lr = ld_peer(ml + kTile + row, r);
+        if (lr == 0.f) continue;  // the share saw no key (its sum says so: NaN scores leave the maximum at -inf too)
+        const float w = mr == -INFINITY ? 1.f : exp2f(mr - mx);
+        sum = fmaf(w, lr, sum);
         const float4 x = ld_peer4(o_s + row * PT + c, r);
         acc.x = fmaf(w, x.x, acc.x), acc.y = fmaf(w, x.y, acc.y), acc.z = fmaf(w, x.z, acc.z), acc.w = fmaf(w, x.w, acc.w);
       }

@@ -703,3 +703,24 @@ def test_f32_attention_tiles_and_shares(B, T, Tk, H, Hkv, D, kw):
     got, glse, want, wlse = run_case(q, k, v, O.F32, lse=True, **kw)
     assert ops.chosen() == "attention: graph dtype"
     assert np.isfinite(got).all() and max_abs(got, want) < 1e-4 and max_abs(glse, wlse) < 1e-4
+
+
+@pytest.mark.parametrize("dt", [O.F32, O.BF16])
+@pytest.mark.parametrize("B,Tk", [(1, 1030), (80, 130)])
+def test_a_nan_query_row_stays_nan_whether_or_not_its_keys_are_shared(dt, B, Tk):
+    """Keys shared over a cluster (one lane) and not (many): NaN scores are no empty share.
+    Every other row is what it is without the NaN."""
+    T, H, D = 16 if dt == O.F32 else 2, 4, 64
+    rng = np.random.default_rng(Tk)
+    q, k, v = (dev(normal(rng, s, 1.0, dt), dt) for s in ((B, T, H, D), (B, Tk, H, D), (B, Tk, H, D)))
+    lens = torch.full((B,), Tk - 1, dtype=torch.int32).cuda()
+    a = ops.Attn(keys=ops.KeyMask.Lens(lens), want_lse=True)
+    want, wlse = ops.attention(q, k, v, a)
+    q[0, 1, 2, 5] = float("nan")
+    got, lse = ops.attention(q, k, v, a)
+    ops.device_status()
+    hit = torch.zeros(B, T, H, dtype=torch.bool).cuda()
+    hit[0, 1, 2] = True
+    assert torch.isnan(got[hit]).all() and torch.equal(got[~hit], want[~hit])
+    hit = hit.transpose(1, 2)
+    assert torch.isnan(lse[hit]).all() and torch.equal(lse[~hit], wlse[~hit])
