@@ -177,8 +177,11 @@ __global__ void __launch_bounds__(kThreadsDec, (DecCfg<D, NQ>::kPerSm))
   uint64_t* full = bars;
   uint64_t* empty = full + S;
   uint64_t* s_full = empty + S;  // [2]
+  // [2], as each of a pair of blocks has its own: with two buffers of weights a softmax warp may
+  // have arrived for block j + 1 before the issuer looks at block j, which on one barrier would
+  // then read as not complete for ever.
   uint64_t* p_full = s_full + 2;
-  uint64_t* pv_done = p_full + 1;  // [2]
+  uint64_t* pv_done = p_full + 2;  // [2]
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(pv_done + 2);
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -246,7 +249,8 @@ __global__ void __launch_bounds__(kThreadsDec, (DecCfg<D, NQ>::kPerSm))
     }
     mbar_init(&s_full[0], 1);
     mbar_init(&s_full[1], 1);
-    mbar_init(p_full, 4);
+    mbar_init(&p_full[0], 4);
+    mbar_init(&p_full[1], 4);
     mbar_init(&pv_done[0], 1);
     mbar_init(&pv_done[1], 1);
     mbar_fence_init();
@@ -314,7 +318,7 @@ __global__ void __launch_bounds__(kThreadsDec, (DecCfg<D, NQ>::kPerSm))
     if (n > 0) scores(0);
     for (int j = 0; j < n && ok; ++j) {
       if (j + 1 < n) scores(j + 1);
-      if (!ok || !mbar_wait(p_full, j & 1, p.status)) break;
+      if (!ok || !mbar_wait(&p_full[j & 1], (j >> 1) & 1, p.status)) break;
       const uint32_t pos = pos_v(j, n);
       const int s = (int)(pos % S);
       if (!mbar_wait(&full[s], (pos / S) & 1, p.status)) break;
@@ -494,7 +498,7 @@ __global__ void __launch_bounds__(kThreadsDec, (DecCfg<D, NQ>::kPerSm))
       fence_proxy_async_smem();
       tc_fence_before();
       __syncwarp();
-      if (lane == 0) mbar_arrive(p_full);
+      if (lane == 0) mbar_arrive(&p_full[j & 1]);
     }
     // ---- this CTA's state: m, l, O (f32) into shared memory ----
     if (n > 0) {
