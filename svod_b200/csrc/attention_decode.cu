@@ -14,8 +14,13 @@
 // with NQ = 16 / 32 / 64 columns for the t * (heads / kv_heads) query rows of a KV
 // head. A softmax thread owns one key: its scores are NQ columns of one tensor-memory
 // lane, so the exponentials are those of real query rows only. The softmax weights go
-// to shared memory as two 16-bit halves (value and remainder, 2*NQ rows of B), so
-// O carries them to 16 bits (bf16) or 22 bits (f16) although the MMA is a 16-bit one.
+// to shared memory as two 16-bit halves (value and remainder, 2*NQ rows of B) with an
+// accumulator each, so O carries them to 16 bits (bf16) or 22 bits (f16) although the MMA
+// is a 16-bit one. f16 has no exponents below 2^-24: its value half is scaled by 2^7 (a
+// weight is at most 2^8, see kRescaleAbove) and its remainder by another 2^11, which keeps
+// 22 bits of a weight down to 2^-21 and 2^-44 of any smaller one: 32768 keys of weight
+// 2.5e-8 beside one of weight 1 keep their 8.2e-4 (unscaled, those in the heavy key's share
+// vanished from O, not from the sum).
 //
 // Work split: a cluster of C CTAs (1..16) takes one (batch lane, KV head); each CTA
 // walks an equal share of that lane's VISIBLE key blocks, and the C partial states
@@ -37,6 +42,7 @@
 // Every mbarrier wait is bounded. A softmax warp whose wait ran out keeps walking the
 // named barriers (nothing in between waits without a limit) and the cluster barriers.
 #include <cuda.h>
+#include <cuda_fp16.h>
 #include <math.h>
 #include <stdio.h>
 
@@ -58,6 +64,12 @@ using namespace fa_parts;
 constexpr int kKeys = 128;  // keys per block: the M of both MMAs
 constexpr int kThreadsDec = 192;
 constexpr int kBox = kKeys * 128;  // bytes of one 64-column box of 128 rows
+
+// Powers of two the halves of a weight are scaled by: value, and the remainder once more.
+template <typename T>
+constexpr float kValueUp = std::is_same<T, __half>::value ? 128.f : 1.f;
+template <typename T>
+constexpr float kRestUp = std::is_same<T, __half>::value ? 2048.f : 1.f;
 
 template <int D, int NQ>
 struct DecCfg {
@@ -469,8 +481,9 @@ __global__ void __launch_bounds__(kThreadsDec, (DecCfg<D, NQ>::kPerSm))
             const float pr = ex2_approx(fmaf(__uint_as_float(sr[c]), sl2, -mu[c]));
             if (NQ > 16) lv[c] += pr;
             else l_lane[c] += pr;
-            hi[c] = Elem<T>::from_f(pr);
-            lo[c] = Elem<T>::from_f(pr - Elem<T>::to_f(hi[c]));
+            const float up = pr * kValueUp<T>;
+            hi[c] = Elem<T>::from_f(up);
+            lo[c] = Elem<T>::from_f((up - Elem<T>::to_f(hi[c])) * kRestUp<T>);
           }
 #pragma unroll
           for (int c = 0; c < W; ++c) {
@@ -521,7 +534,7 @@ __global__ void __launch_bounds__(kThreadsDec, (DecCfg<D, NQ>::kPerSm))
           tmem_ld_cols(o_tmem + NQ + q0, lo);
 #pragma unroll
           for (int c = 0; c < 16; ++c)
-            if (q0 + c < p.rows) op[(q0 + c) * D + tid] = __uint_as_float(sr[c]) + __uint_as_float(lo[c]);
+            if (q0 + c < p.rows) op[(q0 + c) * D + tid] = fmaf(__uint_as_float(lo[c]), 1.f / kRestUp<T>, __uint_as_float(sr[c])) * (1.f / kValueUp<T>);
         }
         if (NQ == 16) break;
       }

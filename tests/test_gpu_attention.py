@@ -724,3 +724,21 @@ def test_a_nan_query_row_stays_nan_whether_or_not_its_keys_are_shared(dt, B, Tk)
     assert torch.isnan(got[hit]).all() and torch.equal(got[~hit], want[~hit])
     hit = hit.transpose(1, 2)
     assert torch.isnan(lse[hit]).all() and torch.equal(lse[~hit], wlse[~hit])
+
+
+@pytest.mark.parametrize("T", [1, 20, 40])  # 16, 32 and 64 query rows a block
+def test_small_f16_weights_beside_appended_rows_stay_in_the_sum(T):
+    """32768 keys of weight e^-17.5 = 2.5e-8, below f16's least value, beside one of weight 1:
+    together they are 8.2e-4 of the result. f32 weights give it to the output's rounding, 2^-11;
+    value and remainder lose 2^-17 of such a weight, ex2 and the sums less."""
+    Tk, D = 32768, 64
+    q = torch.zeros(1, T, 1, D, dtype=torch.float16).cuda()
+    k, v = torch.zeros(1, Tk, 1, D, dtype=torch.float16).cuda(), torch.ones(1, Tk, 1, D, dtype=torch.float16).cuda()
+    q[..., 0] = 8.0  # the scale is 1 / 8: a score is k[0]
+    k[:, 0, :, 0], v[:, 0] = 17.5, 0.0
+    app = (torch.zeros(1, 1, 1, D, dtype=torch.float16).cuda(), torch.ones(1, 1, 1, D, dtype=torch.float16).cuda())
+    lens = torch.full((1,), Tk, dtype=torch.int32).cuda()
+    got = host(ops.attention(q, k, v, ops.Attn(keys=ops.KeyMask.Lens(lens), cache=ops.Cache(0, 1, None, app))))
+    assert "cluster:" in ops.chosen()
+    rest = Tk * math.exp(-17.5)
+    assert np.abs(got / (rest / (1.0 + rest)) - 1.0).max() < 2.0 ** -11 + 2.0 ** -16
