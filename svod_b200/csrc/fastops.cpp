@@ -8,12 +8,16 @@
 // library refuses. Nothing has been launched then: ops.py takes the same call through its
 // general path, which converts or reports it.
 //
+// What torch throws underneath (an allocation that fails, a tensor without storage) comes back
+// as the Python exception it is anywhere else, never through the interpreter's frames.
+//
 // The library's entry points come as addresses (`init`), so that SVODB_LIB_PATH keeps
 // selecting the build that runs.
 #include <Python.h>
 
 #include <ATen/ATen.h>
 #include <c10/cuda/CUDAStream.h>
+#include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/python_variable.h>
 
 #include "svodb.h"
@@ -83,6 +87,7 @@ PyObject* none() {
 
 // linear(x, w, opts)
 PyObject* linear(PyObject*, PyObject* const* args, Py_ssize_t n) {
+  HANDLE_TH_ERRORS
   if (n != 3 || p_linear == nullptr) return none();
   svodb_tensor x{}, w{}, y{}, bias{}, res{}, cos{}, sin{}, qn{}, kn{};
   if (!desc(args[0], x) || !desc(args[1], w) || w.rank != 2 || x.rank < 1) return none();
@@ -143,6 +148,7 @@ PyObject* linear(PyObject*, PyObject* const* args, Py_ssize_t n) {
   desc_of(out, y, x.dtype);
   if (p_linear(&x, &w, &o, &y, stream()) != SVODB_OK) return none();
   return THPVariable_Wrap(std::move(out));
+  END_HANDLE_TH_ERRORS
 }
 
 // The options of an attention. `keep` holds the descriptors the struct points at.
@@ -238,6 +244,7 @@ PyObject* with_lse(at::Tensor&& out, at::Tensor&& lse, bool want) {
 
 // attention(q, k, v, opts)
 PyObject* attention(PyObject*, PyObject* const* args, Py_ssize_t n) {
+  HANDLE_TH_ERRORS
   if (n != 4 || p_attention == nullptr) return none();
   svodb_tensor q{}, k{}, v{}, y{};
   if (!desc(args[0], q) || !desc(args[1], k) || !desc(args[2], v) || q.rank != 4) return none();
@@ -251,10 +258,12 @@ PyObject* attention(PyObject*, PyObject* const* args, Py_ssize_t n) {
   if (want) lse = lse_for(qt, q.shape[0], q.shape[2], q.shape[1], o, keep);
   if (p_attention(&q, &k, &v, &o, &y, stream()) != SVODB_OK) return none();
   return with_lse(std::move(out), std::move(lse), want);
+  END_HANDLE_TH_ERRORS
 }
 
 // attention_packed(qkv, heads, kv_heads, opts)
 PyObject* attention_packed(PyObject*, PyObject* const* args, Py_ssize_t n) {
+  HANDLE_TH_ERRORS
   if (n != 4 || p_attention_packed == nullptr) return none();
   svodb_tensor x{}, y{};
   if (!desc(args[0], x) || x.rank != 3) return none();
@@ -271,10 +280,12 @@ PyObject* attention_packed(PyObject*, PyObject* const* args, Py_ssize_t n) {
   if (want) lse = lse_for(xt, x.shape[0], heads, x.shape[1], o, keep);
   if (p_attention_packed(&x, (int32_t)heads, (int32_t)kv, &o, &y, stream()) != SVODB_OK) return none();
   return with_lse(std::move(out), std::move(lse), want);
+  END_HANDLE_TH_ERRORS
 }
 
 // norm(x, residual | None, w, b | None, eps, layer): the norm, or (sum, norm) with a residual
 PyObject* norm(PyObject*, PyObject* const* args, Py_ssize_t n) {
+  HANDLE_TH_ERRORS
   if (n != 6 || p_layer_norm == nullptr) return none();
   svodb_tensor x{}, r{}, w{}, b{}, y{}, s{};
   if (!desc(args[0], x) || !desc(args[2], w)) return none();
@@ -302,6 +313,7 @@ PyObject* norm(PyObject*, PyObject* const* args, Py_ssize_t n) {
   Py_XDECREF(a);
   Py_XDECREF(c);
   return t;
+  END_HANDLE_TH_ERRORS
 }
 
 // init(address of svodb_linear, svodb_attention, svodb_attention_packed, svodb_layer_norm,

@@ -239,3 +239,18 @@ def test_a_cache_row_map_entry_outside_the_cache_is_reported_not_followed():
     assert code(ops.device_status) == L.ERR_SHAPE
     assert torch.equal(bad[0], good[0]) and float(bad[1].abs().max()) == 0.0
     ops.device_status()
+
+
+def test_a_result_the_allocator_refuses_raises_out_of_memory():
+    """The operands are one row seen many times over (stride 0); the result would be
+    petabytes. The caller can catch it and go on."""
+    one = torch.zeros(1, 64, **bf)
+    x, w = one.expand(1 << 44, 64), torch.zeros(32, 64, **bf)
+    with pytest.raises(torch.OutOfMemoryError):
+        ops.linear(x, w)
+    q = torch.zeros(1, 1, 2, 64, **bf).expand(1 << 42, 1, 2, 64)
+    with pytest.raises(torch.OutOfMemoryError):
+        ops.attention(q, q, q)
+    with pytest.raises(torch.OutOfMemoryError):
+        ops.attention_packed(torch.zeros(1, 1, 384, **bf).expand(1 << 42, 1, 384), 2, 2)
+    assert ops.linear(one, w).shape == (1, 32)
