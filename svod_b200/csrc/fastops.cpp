@@ -80,6 +80,16 @@ void desc_of(const at::Tensor& t, svodb_tensor& d, int dtype) {
 
 void* stream() { return (void*)c10::cuda::getCurrentCUDAStream().stream(); }
 
+// A library call with the interpreter let go, as ctypes does it: a launch waits while the
+// device's queue is full, and other Python threads run on meanwhile.
+template <typename F>
+int unlocked(F&& call) {
+  PyThreadState* state = PyEval_SaveThread();
+  const int rc = call();
+  PyEval_RestoreThread(state);
+  return rc;
+}
+
 PyObject* none() {
   PyErr_Clear();
   Py_RETURN_NONE;
@@ -146,7 +156,8 @@ PyObject* linear(PyObject*, PyObject* const* args, Py_ssize_t n) {
   shape[x.rank - 1] = o.gated ? w.shape[0] / 2 : w.shape[0];
   at::Tensor out = at::empty(at::IntArrayRef(shape, x.rank), xt.options());
   desc_of(out, y, x.dtype);
-  if (p_linear(&x, &w, &o, &y, stream()) != SVODB_OK) return none();
+  void* st = stream();
+  if (unlocked([&] { return p_linear(&x, &w, &o, &y, st); }) != SVODB_OK) return none();
   return THPVariable_Wrap(std::move(out));
   END_HANDLE_TH_ERRORS
 }
@@ -256,7 +267,8 @@ PyObject* attention(PyObject*, PyObject* const* args, Py_ssize_t n) {
   at::Tensor out = at::empty(qt.sizes(), qt.options()), lse;
   desc_of(out, y, q.dtype);
   if (want) lse = lse_for(qt, q.shape[0], q.shape[2], q.shape[1], o, keep);
-  if (p_attention(&q, &k, &v, &o, &y, stream()) != SVODB_OK) return none();
+  void* st = stream();
+  if (unlocked([&] { return p_attention(&q, &k, &v, &o, &y, st); }) != SVODB_OK) return none();
   return with_lse(std::move(out), std::move(lse), want);
   END_HANDLE_TH_ERRORS
 }
@@ -278,7 +290,8 @@ PyObject* attention_packed(PyObject*, PyObject* const* args, Py_ssize_t n) {
   at::Tensor out = at::empty({x.shape[0], x.shape[1], heads, d}, xt.options()), lse;
   desc_of(out, y, x.dtype);
   if (want) lse = lse_for(xt, x.shape[0], heads, x.shape[1], o, keep);
-  if (p_attention_packed(&x, (int32_t)heads, (int32_t)kv, &o, &y, stream()) != SVODB_OK) return none();
+  void* st = stream();
+  if (unlocked([&] { return p_attention_packed(&x, (int32_t)heads, (int32_t)kv, &o, &y, st); }) != SVODB_OK) return none();
   return with_lse(std::move(out), std::move(lse), want);
   END_HANDLE_TH_ERRORS
 }
@@ -303,8 +316,11 @@ PyObject* norm(PyObject*, PyObject* const* args, Py_ssize_t n) {
     desc_of(sum, s, x.dtype);
   }
   const svodb_tensor* bp = bias ? &b : nullptr;
-  const int rc = layer ? (res ? p_add_layer_norm(&x, &r, &w, bp, eps, &s, &y, stream()) : p_layer_norm(&x, &w, bp, eps, &y, stream()))
-                       : (res ? p_add_rms_norm(&x, &r, &w, eps, &s, &y, stream()) : p_rms_norm(&x, &w, eps, &y, stream()));
+  void* st = stream();
+  const int rc = unlocked([&] {
+    if (layer) return res ? p_add_layer_norm(&x, &r, &w, bp, eps, &s, &y, st) : p_layer_norm(&x, &w, bp, eps, &y, st);
+    return res ? p_add_rms_norm(&x, &r, &w, eps, &s, &y, st) : p_rms_norm(&x, &w, eps, &y, st);
+  });
   if (rc != SVODB_OK) return none();
   if (!res) return THPVariable_Wrap(std::move(out));
   PyObject* a = THPVariable_Wrap(std::move(sum));

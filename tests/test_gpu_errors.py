@@ -254,3 +254,39 @@ def test_a_result_the_allocator_refuses_raises_out_of_memory():
     with pytest.raises(torch.OutOfMemoryError):
         ops.attention_packed(torch.zeros(1, 1, 384, **bf).expand(1 << 42, 1, 384), 2, 2)
     assert ops.linear(one, w).shape == (1, 32)
+
+
+def test_other_python_threads_run_while_a_call_waits(tmp_path):
+    """Every entry point of the compiled call path replaced by one that sleeps, as a launch does
+    while the device's queue is full."""
+    import subprocess
+    import threading
+    import time
+    (tmp_path / "nap.c").write_text("#include <unistd.h>\nint nap(void) { usleep(400000); return 0; }\n")
+    subprocess.run(["gcc", "-shared", "-fPIC", str(tmp_path / "nap.c"), "-o", str(tmp_path / "nap.so")], check=True)
+    nap = C.cast(C.CDLL(str(tmp_path / "nap.so")).nap, C.c_void_p).value
+    x, w, q, n = torch.zeros(4, 64, **bf), torch.zeros(32, 64, **bf), torch.zeros(1, 4, 2, 64, **bf), torch.ones(64, **bf)
+    fast = L.fastops()
+    ticks, stop = [0], threading.Event()
+
+    def tick():
+        while not stop.wait(0.005):
+            ticks[0] += 1
+
+    other = threading.Thread(target=tick)
+    try:
+        fast.init(*[nap] * 7)
+        other.start()
+        for call in (lambda: fast.linear(x, w, None), lambda: fast.attention(q, q, q, None),
+                     lambda: fast.attention_packed(torch.zeros(1, 4, 384, **bf), 2, 2, None),
+                     lambda: fast.norm(x, None, n, None, 1e-5, True)):
+            before, t = ticks[0], time.monotonic()
+            assert call() is not None and time.monotonic() - t > 0.3
+            assert ticks[0] - before > 10
+    finally:
+        stop.set()
+        other.join()
+        L._fast = None
+        ops._call = None
+        L.fastops()  # bound to the library again
+    assert ops.linear(x, w).shape == (4, 32) and ops.chosen().startswith("linear")
