@@ -240,24 +240,36 @@ _lib = None
 _fast = None
 
 
+class _NoFastOps:
+    """In the place of the compiled call path where it is not built: every call goes the general way."""
+
+    def __getattr__(self, name):
+        return lambda *args: None
+
+
 def fastops():
     """The compiled call path (csrc/fastops.cpp), bound to this library's entry points."""
     global _fast
     if _fast is None:
         import importlib.machinery
         import importlib.util
+        import warnings
 
-        import torch  # noqa: F401 — its libraries carry the symbols the module uses
+        import torch  # its libraries carry the symbols the module uses
         path = Path(__file__).resolve().parent / "lib" / "_fastops.so"
-        if not path.exists():
-            raise RuntimeError(f"{path} is missing: build it with `python -m svod_b200.build`")
-        loader = importlib.machinery.ExtensionFileLoader("_fastops", str(path))
-        mod = importlib.util.module_from_spec(importlib.util.spec_from_file_location("_fastops", str(path), loader=loader))
-        loader.exec_module(mod)
-        lib = load()
-        mod.init(*[C.cast(getattr(lib, f"svodb_{n}"), C.c_void_p).value for n in (
-            "linear", "attention", "attention_packed", "layer_norm", "rms_norm", "add_layer_norm", "add_rms_norm")])
-        _fast = mod
+        try:
+            loader = importlib.machinery.ExtensionFileLoader("_fastops", str(path))
+            mod = importlib.util.module_from_spec(importlib.util.spec_from_file_location("_fastops", str(path), loader=loader))
+            loader.exec_module(mod)
+            if mod.torch != torch.__version__:
+                raise ImportError(f"{path} was built for torch {mod.torch}, this is {torch.__version__}")
+            lib = load()
+            mod.init(*[C.cast(getattr(lib, f"svodb_{n}"), C.c_void_p).value for n in (
+                "linear", "attention", "attention_packed", "layer_norm", "rms_norm", "add_layer_norm", "add_rms_norm")])
+            _fast = mod
+        except ImportError as e:
+            warnings.warn(f"ops take 15-30 us a call longer than need be: {e}; build with `python -m svod_b200.build`")
+            _fast = _NoFastOps()
     return _fast
 
 

@@ -21,6 +21,7 @@ LIB = OUT_DIR / "libsvodb.so"
 FAST = OUT_DIR / "_fastops.so"  # the op layer's Python call path (csrc/fastops.cpp)
 
 NVCC = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")
+CXX = os.environ.get("CXX", "g++")
 FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a",
     "-lineinfo", "-O3", "-std=c++17",
@@ -53,29 +54,45 @@ def _compile(src: Path, verbose: bool) -> Path:
 
 def _build_fast() -> None:
     """The CPython module against torch's headers; its torch symbols are those of the
-    libraries `import torch` has loaded."""
+    libraries `import torch` has loaded, so another torch or Python builds it anew."""
     src = CSRC / "fastops.cpp"
     stamp = max(src.stat().st_mtime, (INCLUDE / "svodb.h").stat().st_mtime)
-    if FAST.exists() and FAST.stat().st_mtime >= stamp:
-        return
     import sysconfig
+    from importlib import metadata
+    against = f"{metadata.version('torch')} {sysconfig.get_config_var('SOABI')}"
+    built = FAST.with_suffix(".built")
+    if FAST.exists() and FAST.stat().st_mtime >= stamp and built.exists() and built.read_text() == against:
+        return
 
     import torch
     inc = Path(torch.__file__).resolve().parent / "include"
-    cmd = ["g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-w", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+    cmd = [CXX, "-O2", "-std=c++17", "-fPIC", "-shared", "-w", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+           f'-DSVODB_TORCH="{torch.__version__}"',
            f"-I{INCLUDE}", f"-I{inc}", f"-I{inc}/torch/csrc/api/include", f"-I{sysconfig.get_paths()['include']}",
            f"-I{Path(NVCC).parent.parent}/include", str(src), "-o", str(FAST), f"-L{inc.parent}/lib", "-ltorch_python", "-ltorch_cpu",
            "-lc10", "-lc10_cuda"]
     r = subprocess.run(cmd, capture_output=True, text=True)
     if r.returncode != 0:
-        raise RuntimeError(f"g++ failed for {src.name}:\n{r.stdout}\n{r.stderr}")
+        raise RuntimeError(f"{CXX} failed for {src.name}:\n{r.stdout}\n{r.stderr}")
+    built.write_text(against)
+
+
+def _try_build_fast() -> None:
+    """The library is whole without the module, and a user of the C library needs neither
+    torch's headers nor Python's: what keeps it from being built is said, not raised. One
+    that is there and could not be brought up to date goes, so that nothing loads it."""
+    try:
+        _build_fast()
+    except Exception as e:
+        FAST.unlink(missing_ok=True)
+        print(f"svod_b200.build: without {FAST.name} (ops take the ctypes path): {e}", file=sys.stderr)
 
 
 def build(verbose: bool = False) -> Path:
     OBJ_DIR.mkdir(parents=True, exist_ok=True)
     srcs = sorted(CSRC.glob("*.cu"))
     with ThreadPoolExecutor(max_workers=min(8, len(srcs) + 1)) as ex:
-        fast = ex.submit(_build_fast)
+        fast = ex.submit(_try_build_fast)
         objs = list(ex.map(lambda s: _compile(s, verbose), srcs))
     fast.result()
     if not LIB.exists() or any(o.stat().st_mtime > LIB.stat().st_mtime for o in objs):

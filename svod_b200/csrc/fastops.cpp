@@ -360,4 +360,8 @@ PyModuleDef kModule = {PyModuleDef_HEAD_INIT, "_fastops", "compiled call path of
 
 }  // namespace
 
-PyMODINIT_FUNC PyInit__fastops(void) { return PyModule_Create(&kModule); }
+PyMODINIT_FUNC PyInit__fastops(void) {
+  PyObject* m = PyModule_Create(&kModule);
+  if (m != nullptr) PyModule_AddStringConstant(m, "torch", SVODB_TORCH);  // the torch it was built for
+  return m;
+}

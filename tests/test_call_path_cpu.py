@@ -33,3 +33,39 @@ with FakeTensorMode():
 def test_what_torch_throws_is_raised():
     r = subprocess.run([sys.executable, "-c", SCRIPT], cwd=ROOT, capture_output=True, text=True)
     assert r.returncode == 0 and r.stdout.split() == ["raised"] * 4, (r.returncode, r.stderr[-500:])
+
+
+def test_the_library_builds_and_the_ops_work_without_the_compiled_call_path(tmp_path, monkeypatch, capsys):
+    from svod_b200 import _lib, build, ops
+    monkeypatch.setattr(build, "FAST", tmp_path / "_fastops.so")
+    monkeypatch.setattr(build, "CXX", "false")  # no headers, no compiler: whatever keeps it from being built
+    build.FAST.write_bytes(b"an older build")
+    assert build.build() == build.LIB
+    assert not build.FAST.exists() and "_fastops.so" in capsys.readouterr().err
+    # the ops then go the general way: its checks, its errors
+    monkeypatch.setattr(_lib, "_fast", None)
+    monkeypatch.setattr(ops, "_call", None)
+    monkeypatch.setattr(_lib, "__file__", str(tmp_path / "_lib.py"))
+    with pytest.warns(UserWarning, match="svod_b200.build"), pytest.raises(ops.OpsError) as e:
+        ops.linear(torch.zeros(2, 4), torch.zeros(3, 4))
+    assert e.value.kind == "Unrealized"
+
+
+def test_another_torch_builds_the_call_path_anew(tmp_path, monkeypatch):
+    from importlib import metadata
+    from svod_b200 import build
+    monkeypatch.setattr(build, "FAST", tmp_path / "_fastops.so")
+    ran = []
+
+    def compiler(cmd, **kw):
+        ran.append(cmd)
+        build.FAST.write_bytes(b"built")
+        return subprocess.CompletedProcess(cmd, 0, "", "")
+
+    monkeypatch.setattr(build.subprocess, "run", compiler)
+    build._build_fast()
+    build._build_fast()
+    assert len(ran) == 1
+    monkeypatch.setattr(metadata, "version", lambda name: "0.0.1")
+    build._build_fast()
+    assert len(ran) == 2
