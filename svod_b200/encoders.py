@@ -80,8 +80,10 @@ def _randn(gen, shape, dtype, device, sigma=0.02):
 def _over_real_rows(ids: torch.Tensor, aux: torch.Tensor, run):
     """`run(aux)` over the batch's rows without their trailing padding where that pays
     and every op of the stack has a kernel for it, over the padded batch otherwise.
-    `aux`: the padding mask `[B, L]` or the lengths `[B]`."""
-    if aux.shape[0] == ids.shape[0] and ops.rows_pay(*ids.shape):
+    `aux`: the padding mask `[B, L]` or the lengths `[B]`. A floating mask stays with the
+    padded batch: attention takes its nonzero values, the pooling its integer parts, and
+    packed rows have one mask for both."""
+    if not aux.is_floating_point() and aux.shape[0] == ids.shape[0] and ops.rows_pay(*ids.shape):
         try:
             with ops.PackedRows(aux, ids.shape[1]) as rows:
                 return run(aux if rows.mask is None else rows.mask)

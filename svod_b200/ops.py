@@ -518,8 +518,10 @@ class PackedRows:
         batch = aux.shape[0]
         self.given = length
         self.length = -(-length // 64) * 64
-        if aux.dim() == 1 or aux.dtype not in (torch.bool, torch.uint8, torch.int32):
+        if aux.dim() == 1:
             aux = aux.to(torch.int32)
+        elif aux.dtype not in (torch.bool, torch.uint8, torch.int32):
+            aux = aux != 0  # nonzero where attended (`KeyMask`), not what an integer conversion leaves of it
         self.aux = aux.contiguous()
         self.mask = (torch.empty(batch, self.length, dtype=torch.uint8, device=aux.device) if aux.dim() == 2 else None)
         self.table = torch.zeros(L.load().svodb_rows_table_bytes(batch, length) // 4, dtype=torch.int32, device=aux.device)

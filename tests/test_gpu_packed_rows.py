@@ -91,6 +91,21 @@ def test_masks_with_holes_and_empty_rows(kind, pooling, dtype, monkeypatch):
     assert (got[1] == want[1]).all() or pooling == "cls"
 
 
+@pytest.mark.parametrize("pooling", ["cls", "mean"])
+@pytest.mark.parametrize("value", [0.5, 1 << 32])
+def test_masks_of_another_type_attend_where_they_are_nonzero(value, pooling, monkeypatch):
+    from svod_b200 import ops
+    model = _model("modernbert")
+    model.cfg.pooling = pooling
+    ids, mask = _batch([300, 129, 64, 200], 300, "modernbert")
+    aux = mask.to(torch.float32 if value < 1 else torch.int64)
+    aux[:, 20:60] *= value  # an integer conversion would leave 0 of it
+    got = model.forward(ids, aux)
+    monkeypatch.setattr(ops, "rows_pay", lambda b, n: False)
+    # (the pooling of a padded batch converts to i32, so the mean of the int64 case has no reference there)
+    _close(got, model.forward(ids, mask if value > 1 else aux), "modernbert")
+
+
 def test_lengths_outside_the_row(monkeypatch):
     from svod_b200 import ops
     model = _model("qwen3")
