@@ -338,6 +338,9 @@ int svodb_norm_pool(const svodb_tensor* hidden, const svodb_tensor* norm_w, cons
 size_t svodb_rows_table_bytes(int64_t batch, int64_t len);
 /* Whether the library's own stacks run a plan [batch, len] that way. */
 int svodb_rows_pay(int64_t batch, int64_t len);
+/* Whether every op of a stack with this hidden width and head width has a kernel over packed
+ * rows (operands on the 16-byte grid); `placed`: its projections rotate or norm heads. */
+int svodb_rows_take(int64_t hidden, int32_t head_dim, int32_t placed);
 int svodb_rows_begin(const svodb_tensor* mask_or_lengths, int64_t len, void* table, svodb_tensor* mask_out, void* stream);
 void svodb_rows_end(void);
 

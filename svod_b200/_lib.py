@@ -205,6 +205,7 @@ SYMBOLS = [
     ("svodb_norm_pool", C.c_int, [TensorP, TensorP, TensorP, C.c_double, C.c_int32, TensorP, TensorP, C.c_int32,
                                   C.c_int32, TensorP, C.c_void_p]),
     ("svodb_rows_pay", C.c_int, [C.c_int64, C.c_int64]),
+    ("svodb_rows_take", C.c_int, [C.c_int64, C.c_int32, C.c_int32]),
     ("svodb_rows_table_bytes", C.c_size_t, [C.c_int64, C.c_int64]),
     ("svodb_rows_begin", C.c_int, [TensorP, C.c_int64, C.c_void_p, TensorP, C.c_void_p]),
     ("svodb_rows_end", None, []),

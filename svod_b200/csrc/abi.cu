@@ -903,6 +903,14 @@ size_t svodb_rows_table_bytes(int64_t batch, int64_t len) {
 // Below 1024 padded rows a stack is bound by its launches, not by its rows.
 int svodb_rows_pay(int64_t batch, int64_t len) { return batch > 0 && len > 0 && batch * len >= 1024 ? 1 : 0; }
 
+// What would be refused behind the whole stack (the fused final norm and pooling: whole spans of
+// 256 columns up to 2048) or in its first layer (attention's tiles, heads turned in the store).
+int svodb_rows_take(int64_t hidden, int32_t head_dim, int32_t placed) {
+  if (hidden <= 0 || hidden % 256 != 0 || hidden > 2048) return 0;
+  if (placed) return head_dim == 64 || head_dim == 128 ? 1 : 0;
+  return head_dim > 0 && head_dim % 8 == 0 && head_dim <= 128 ? 1 : 0;
+}
+
 int svodb_rows_begin(const svodb_tensor* mask_or_lengths, int64_t len, void* table, svodb_tensor* mask_out, void* stream) {
   static const char* OP = "rows_begin";
   GUARD(OP);

@@ -484,7 +484,8 @@ int svodb_model_plan(svodb_model* m, int64_t rows, int64_t len, int32_t referenc
   p->pooled = (float*)b.take((size_t)rows * D * 4);
   p->table = b.take(table_bytes);
   p->mask = (uint8_t*)b.take((size_t)rows * padded_len(len));
-  p->packed = !reference_ops && svodb_rows_pay(rows, len);
+  const int32_t hd = m->kind == kQwen3 ? m->q.head_dim : m->kind == kXlmr ? m->x.hidden / m->x.heads : m->m.hidden / m->m.heads;
+  p->packed = !reference_ops && svodb_rows_pay(rows, len) && svodb_rows_take(D, hd, m->kind != kXlmr);
   Acts a = carve(b, *m, rows, padded_len(len), reference_ops);
   const int64_t table_len = tensor_len(p);
   cudaMemsetAsync(p->table, 0, table_bytes, p->stream);

@@ -77,16 +77,30 @@ def _randn(gen, shape, dtype, device, sigma=0.02):
     return (torch.randn(shape, generator=gen, device=device, dtype=torch.float32) * sigma).to(dtype)
 
 
-def _over_real_rows(ids: torch.Tensor, aux: torch.Tensor, run):
+def _over_real_rows(model, ids: torch.Tensor, aux: torch.Tensor, out, head_dim: int, placed: bool, run):
     """`run(aux)` over the batch's rows without their trailing padding where that pays
     and every op of the stack has a kernel for it, over the padded batch otherwise.
     `aux`: the padding mask `[B, L]` or the lengths `[B]`. A floating mask stays with the
     padded batch: attention takes its nonzero values, the pooling its integer parts, and
-    packed rows have one mask for both."""
-    if not aux.is_floating_point() and aux.shape[0] == ids.shape[0] and ops.rows_pay(*ids.shape):
+    packed rows have one mask for both.
+
+    A stack of a width without such kernels, or whose result lies off the 16-byte grid, is not
+    begun. One that an op refuses all the same
+    (a weight off the 16-byte grid) has run in part for nothing: the model remembers the shape,
+    so that a capture behind an eager run holds the padded stack alone."""
+    shape = tuple(ids.shape)
+    refused = model.__dict__.setdefault("_padded_shapes", set())
+    if (not aux.is_floating_point() and aux.shape[0] == shape[0] and shape not in refused and ops.rows_pay(*shape)
+            and (out is None or (out.data_ptr() % 16 == 0 and out.stride(0) % 4 == 0))
+            and ops.rows_take(model.cfg.hidden_size, head_dim, placed)):
         try:
-            with ops.PackedRows(aux, ids.shape[1]) as rows:
-                return run(aux if rows.mask is None else rows.mask)
+            with ops.PackedRows(aux, shape[1]) as rows:
+                try:
+                    return run(aux if rows.mask is None else rows.mask)
+                except ops.OpsError as e:
+                    if e.code == ops.ERR_UNSUPPORTED:
+                        refused.add(shape)
+                    raise
         except ops.OpsError as e:
             if e.code != ops.ERR_UNSUPPORTED:
                 raise
@@ -147,14 +161,15 @@ class XlmRobertaEncoder:
         return x
 
     def forward(self, ids, mask, out=None, gather=None):
-        mode = ops.POOL_CLS if self.cfg.pooling == "cls" else ops.POOL_MEAN
+        c = self.cfg
+        mode = ops.POOL_CLS if c.pooling == "cls" else ops.POOL_MEAN
 
         def run(mask):
             h = self.hidden(ids, mask)
             # post-LN stack: the last layer's norm is the final one; pooling + L2 in one kernel
             return ops.norm_pool(h, aux=mask if mode == ops.POOL_MEAN else None, mode=mode, out=out, gather=gather)
 
-        return _over_real_rows(ids, mask, run)
+        return _over_real_rows(self, ids, mask, out, c.hidden_size // c.num_attention_heads, False, run)
 
 
 # --------------------------------------------------------------------------- Qwen3
@@ -225,7 +240,9 @@ class Qwen3Embedder:
             return ops.norm_pool(x, self.p["norm_w"], None, self.cfg.rms_norm_eps, layer=False, aux=lengths,
                                  mode=ops.POOL_LAST, out=out, gather=gather)
 
-        return _over_real_rows(ids, lengths, run) if self.fused_prologue else run(lengths)
+        if not self.fused_prologue:
+            return run(lengths)
+        return _over_real_rows(self, ids, lengths, out, self.cfg.head_dim, True, run)
 
 
 # --------------------------------------------------------------------------- ModernBERT
@@ -298,7 +315,7 @@ class ModernBertEncoder:
             return ops.norm_pool(x, p["final_ln_w"], None, c.norm_eps, aux=mask if mode == ops.POOL_MEAN else None,
                                  mode=mode, out=out, gather=gather)
 
-        return _over_real_rows(ids, mask, run)
+        return _over_real_rows(self, ids, mask, out, c.hidden_size // c.num_attention_heads, True, run)
 
 
 # --------------------------------------------------------------------------- plan replay

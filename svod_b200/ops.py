@@ -550,6 +550,12 @@ def rows_pay(batch: int, length: int) -> bool:
     return bool(L.load().svodb_rows_pay(batch, length))
 
 
+def rows_take(hidden: int, head_dim: int, placed: bool) -> bool:
+    """Whether every op of a stack of this width has a kernel over packed rows; `placed`:
+    its projections rotate or norm heads."""
+    return bool(L.load().svodb_rows_take(hidden, head_dim, int(placed)))
+
+
 # ----------------------------------------------------------------------------- glue
 def embed(ids, table, pos_table=None, type_row=None, pad_id: int = -1):
     """Token embedding lookup; with `pos_table` and `pad_id >= 0` the XLM-R

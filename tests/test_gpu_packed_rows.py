@@ -156,3 +156,44 @@ def test_calls_without_a_kernel_fall_back():
             ops.heads(torch.empty(4, 256, 960, dtype=torch.bfloat16, device="cuda"), ops.Qkv(10, 10, 32))
     assert e.value.code == ops.ERR_UNSUPPORTED
     assert ops._packed.length is None
+
+
+@pytest.mark.parametrize("hidden,heads,off", [(384, 12, ""), (2304, 18, ""), (512, 8, "out"), (512, 8, "weight")])
+def test_a_stack_without_kernels_for_it_runs_once(hidden, heads, off, monkeypatch):
+    """Widths the fused pooling does not take and a result off the 16-byte grid (nothing of the
+    packed stack is launched), and a final norm's weight off it, which only the last op sees (the
+    second run knows): launches of an eager run and of a captured plan."""
+    from svod_b200 import encoders as E
+    from svod_b200 import native, ops
+    kind = "modernbert" if off == "weight" else "xlmr"
+    if kind == "xlmr":
+        cfg = E.XlmRobertaConfig(vocab_size=500, hidden_size=hidden, num_hidden_layers=2, num_attention_heads=heads,
+                                 intermediate_size=512, max_position_embeddings=300)
+        model = E.XlmRobertaEncoder.random_init(cfg, seed=2)
+    else:
+        model = _model(kind, hidden)
+        model.p["final_ln_w"] = torch.ones(hidden + 1, dtype=model.cfg.dtype, device="cuda")[1:]
+    ids, mask = _batch([200, 100, 256, 33], 256, kind)
+    out = torch.empty(4 * hidden + 1, device="cuda")[1:].view(4, hidden) if off == "out" else None
+
+    def launches(call):
+        before = ops.launches
+        call()
+        return ops.launches - before
+
+    with monkeypatch.context() as m:
+        m.setattr(ops, "rows_pay", lambda b, n: False)
+        want = model.forward(ids, mask).clone()
+        once = launches(lambda: model.forward(ids, mask, out))
+    assert ops.rows_pay(*ids.shape)
+    first = launches(lambda: model.forward(ids, mask, out))
+    assert first > once if off == "weight" else first == once
+    assert launches(lambda: model.forward(ids, mask, out)) == once
+    plan = E.Plan(model, 4, 256, "mask", out=out if out is not None else torch.empty(4, hidden, device="cuda"))
+    assert launches(plan.capture) == 2 * once  # the eager run and the captured one
+    host_out = torch.empty(4, hidden).pin_memory()
+    plan.run(ids.cpu().pin_memory(), mask.cpu().pin_memory(), host_out)
+    plan.check()
+    _close(host_out, want, kind)
+    got = (native.NativeXlmRoberta if kind == "xlmr" else native.NativeModernBert)(model).run(ids.cpu().numpy(), mask.cpu().numpy().astype(np.uint8))
+    _close(torch.from_numpy(got), want, kind)
