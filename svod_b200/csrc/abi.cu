@@ -481,6 +481,7 @@ int svodb_linear(const svodb_tensor* x, const svodb_tensor* w, const svodb_linea
     snprintf(key, sizeof key, "gemm|%s|%lld|%lld|%lld|%s%s%s", dtype_name(x->dtype), (long long)a.m, (long long)n,
              (long long)k, epi, opts->residual != nullptr ? "+res" : "", act != SVODB_ACT_NONE ? "+act" : "");
     a.force_bn = config_lookup(key);
+    if (a.force_bn >= kForceSmall && !small_code(a.force_bn)) a.force_bn = 0;  // names nothing: the library's own choice
     if (gemm_tc_covers(a)) snprintf(g_config_key, sizeof g_config_key, "%s", key);
   }
   if (qo != nullptr) {
@@ -500,7 +501,7 @@ int svodb_linear(const svodb_tensor* x, const svodb_tensor* w, const svodb_linea
     f.norm_k_heads = qo->kv_heads;
     f.norm_eps = (float)qo->eps;
     const bool any = f.rope_cos != nullptr || f.norm_q != nullptr || f.norm_k != nullptr;
-    if (any && (f.force_bn == 0 || f.force_bn >= kForceSmall)) {
+    if (any && (f.force_bn == 0 || small_code(f.force_bn))) {
       const int splits = gemm_small_splits(f);
       if (splits > 0) {
         if (launch_gemm_small(f, splits, s, cfg, sizeof cfg) != 0)
@@ -548,7 +549,7 @@ int svodb_linear(const svodb_tensor* x, const svodb_tensor* w, const svodb_linea
       }
     }
   }
-  if (a.force_bn == 0 || a.force_bn >= kForceSmall) {
+  if (a.force_bn == 0 || small_code(a.force_bn)) {
     const int splits = gemm_small_splits(a);
     if (splits > 0) {
       if (launch_gemm_small(a, splits, s, cfg, sizeof cfg) != 0)

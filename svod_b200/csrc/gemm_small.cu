@@ -476,7 +476,7 @@ int run_s(const GemmArgs& a, int splits, cudaStream_t s, char* cfg, size_t cfg_l
 int gemm_small_splits(const GemmArgs& a) {
   if (!gemm_tc_covers(a)) return 0;
   const bool per_head = a.rope_cos != nullptr || a.norm_q != nullptr || a.norm_k != nullptr;
-  if (a.force_bn > kForceSmall && (a.force_bn & 15) <= 8) return a.force_bn - kForceSmall;
+  if (small_code(a.force_bn)) return a.force_bn - kForceSmall;
   const int bn = per_head ? a.rope_head_dim : 64;
   const int out_bn = a.gated ? bn / 2 : bn;
   const int64_t tiles = ((a.m + BM - 1) / BM) * ((a.n + out_bn - 1) / out_bn);

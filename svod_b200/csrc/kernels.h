@@ -261,6 +261,11 @@ struct GemmArgs {
 // accumulator columns, + kSmallWide = of 128 (a per-head store's tile is its head).
 constexpr int kForceSmall = 1024;
 constexpr int kSmallWide = 16;
+// Whether `code` names a form of the few-tile kernel: one to eight CTAs a tile, of either width.
+constexpr bool small_code(int code) {
+  return code > kForceSmall && code < kForceSmall + 2 * kSmallWide && (code & (kSmallWide - 1)) >= 1 &&
+         (code & (kSmallWide - 1)) <= 8;
+}
 // The few-tile kernel: CTAs per tile it would run the call with (+ kSmallWide), 0 where another
 // kernel is the better one.
 int gemm_small_splits(const GemmArgs& a);

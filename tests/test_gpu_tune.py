@@ -76,3 +76,29 @@ def test_decode_attention_splits_come_from_the_store(tmp_path):
         tune.activate(None)
     assert max_abs(got, want) < 2e-2
     assert max_abs(host(ops.attention(Q, K, V, a)), want) < 2e-2  # and without the store
+
+
+def test_a_stored_config_that_names_nothing_is_ignored():
+    """Codes around those of the few-tile kernel (1024 + CTAs a tile 1..8, + 16 for 128 columns):
+    a stale or broken store changes no call."""
+    lib = L.load()
+    lib.svodb_config_clear()
+    dt = O.BF16
+    rng = np.random.default_rng(9)
+    x, w = dev(normal(rng, (128, 1024), 1.0, dt), dt), dev(normal(rng, (1024, 1024), 0.05, dt), dt)
+    want = ops.linear(x, w)
+    own, key = ops.chosen(), lib.svodb_last_config_key()
+    try:
+        for code in (1024, 1033, 1039, 1040, 1049, 1056, 1057, 1088, 2 ** 31 - 1):
+            lib.svodb_config_set(key, code)
+            assert torch.equal(ops.linear(x, w), want) and ops.chosen() == own, code
+        for code, form in ((1025, "bn:64,"), (1032, "cluster:8"), (1042, "bn:128,")):
+            lib.svodb_config_set(key, code)
+            got = ops.linear(x, w)
+            assert form in ops.chosen() and "cluster:" in ops.chosen()
+            # the same f32 sum of K products in another order (each within K * 2^-24 of the sum of their
+            # absolute values), then a rounding to bf16 on either side
+            bound = 2.0 ** -7 * want.double().abs() + 2 * 1024 * 2.0 ** -24 * (x.double().abs() @ w.double().abs().T)
+            assert ((got.double() - want.double()).abs() <= bound).all()
+    finally:
+        lib.svodb_config_clear()
