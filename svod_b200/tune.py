@@ -2,7 +2,7 @@
 (tk/src/tune.rs): the config an op uses for a shape is measured once, kept in
 the process and in a file, and replayed afterwards.
 
-What is stored: the tile width of the tensor-core GEMM per `linear` shape (the
+What is stored: the kernel and tile width of the tensor-core GEMM per `linear` shape (the
 library keeps the process map and reports each call's key,
 `svodb_last_config_key` / `svodb_config_set`) and the key-split count of a
 decode-shaped attention (`Attn.splits = None` asks the store, as the
@@ -24,8 +24,11 @@ from typing import Callable, Dict, Iterable, Optional, Tuple
 
 from . import _lib as L
 
-FORMAT = 1
+FORMAT = 2  # 1: files measured before there was a few-tile kernel (GEMM) or one for few query rows (attention)
 GEMM_WIDTHS = (64, 128, 256, 512)  # 512 = the CTA-pair kernel (256 x 256 tiles on two SMs)
+# The few-tile kernel: 1024 + CTAs a tile, + 16 for tiles of 128 columns.
+FEW_TILE_FORMS = tuple(1024 + wide + ctas for wide in (0, 16) for ctas in (1, 2, 4, 8))
+OWN_CHOICE = 0  # whatever the library picks for the shape
 
 
 def enabled() -> bool:
@@ -132,13 +135,14 @@ class TuneStore:
         return best
 
     def tune_linear(self, x, w, opts=None) -> Optional[int]:
-        """Measures the tile widths for this `linear` shape on a store miss and
-        keeps the winner; returns the width in use (None when the shape runs
-        the generic kernel, which has nothing to choose)."""
+        """Measures the tile widths for this `linear` shape on a store miss — and, where
+        the library runs its few-tile kernel, that choice and the kernel's other forms —
+        and keeps the winner; returns the value in use (None when the shape runs the
+        generic kernel, which has nothing to choose)."""
         from . import ops
         lib = L.load()
         ops.linear(x, w, opts)
-        key = lib.svodb_last_config_key().decode()
+        key, few_tiles = lib.svodb_last_config_key().decode(), "cluster:" in ops.chosen()
         if not key:
             return None
         if self.get(key) is not None or not enabled():
@@ -152,9 +156,14 @@ class TuneStore:
             # a choice the shape or the epilogue cannot take is ignored by the library
             run(bn)
             chosen = ops.chosen()
+            if bn == OWN_CHOICE:
+                return True
+            if bn in FEW_TILE_FORMS:
+                return f"bn:{128 if bn & 16 else 64}," in chosen and f"cluster:{bn & 15}" in chosen
             return ("cta_pair:1" in chosen) if bn == 512 else (f"bn:{bn}," in chosen and "cta_pair" not in chosen)
 
-        best = self.pick(key, [bn for bn in GEMM_WIDTHS if takes(bn)], run)
+        forms = (OWN_CHOICE, *FEW_TILE_FORMS, *GEMM_WIDTHS) if few_tiles else GEMM_WIDTHS
+        best = self.pick(key, [bn for bn in forms if takes(bn)], run)
         lib.svodb_config_set(key.encode(), best)
         return best
 

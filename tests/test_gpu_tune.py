@@ -102,3 +102,25 @@ def test_a_stored_config_that_names_nothing_is_ignored():
             assert ((got.double() - want.double()).abs() <= bound).all()
     finally:
         lib.svodb_config_clear()
+
+
+def test_tuning_a_few_tile_projection_keeps_its_kernel(tmp_path):
+    """128 x 1024 x 4096 takes less than half the time on the few-tile kernel: tuning offers the
+    library's own choice and the kernel's forms beside the tile widths."""
+    lib = L.load()
+    lib.svodb_config_clear()
+    x, w = torch.randn(128, 4096, device="cuda").bfloat16(), torch.randn(1024, 4096, device="cuda").bfloat16()
+    try:
+        store = tune.TuneStore(torch.cuda.get_device_name(0), directory=tmp_path)
+        best = store.tune_linear(x, w)
+        assert best == tune.OWN_CHOICE or best in tune.FEW_TILE_FORMS
+        ops.linear(x, w)
+        assert "cluster:" in ops.chosen()
+        lib.svodb_config_clear()
+        again = tune.TuneStore(torch.cuda.get_device_name(0), directory=tmp_path)
+        assert again.load() == 1 and again.tune_linear(x, w) == best
+        # a file from before the kernel holds widths that shut it out: not read
+        again.path.write_text(again.path.read_text().replace(f"format {tune.FORMAT}", "format 1"))
+        assert tune.TuneStore(torch.cuda.get_device_name(0), directory=tmp_path).load() == 0
+    finally:
+        lib.svodb_config_clear()
