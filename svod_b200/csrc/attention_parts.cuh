@@ -77,6 +77,18 @@ struct Range {
   int lo, hi;  // key blocks [lo, hi)
 };
 
+// Blocks in which the two tiles of an item take turns on the MUFU unit: those both have,
+// where their ranges begin near one another (two 128-row tiles under a sliding window are
+// two blocks apart). Tile 0 waits for tile 1's block n before its own n + 1, so the ring has
+// to bring the later range's first block while the earlier range stands at its second: a
+// chunk border or a segment's start inside an item may lie any number of blocks further on,
+// and such an item stood until its bounded waits ran out. Its tiles go their own ways.
+constexpr int kTurnReach = 2;
+__device__ __forceinline__ int paired_blocks(const Range& r0, const Range& r1) {
+  const int apart = r0.lo < r1.lo ? r1.lo - r0.lo : r0.lo - r1.lo;
+  return apart > kTurnReach ? 0 : min(r0.hi - r0.lo, r1.hi - r1.lo);
+}
+
 // The mask context shared by every role of a CTA.
 struct Ctx {
   int64_t len;       // visible key count bound: min(Tk, key_lens[b] or the prefix mask's length)

@@ -381,7 +381,7 @@ __global__ void __launch_bounds__(kThreadsFa, 1)
     // Left alone they fall into step, their exponential bursts collide and the
     // unit idles while both read scores and take maxima. They take turns
     // instead: tile 0 runs the exponentials of its block n, then tile 1 those
-    // of its block n, then tile 0 block n+1, ... for the blocks both tiles have,
+    // of its block n, then tile 0 block n+1, ... for the blocks both tiles have (`paired_blocks`),
     // so one tile's TMEM reads and maxima overlap the other's exponentials.
     // The hand-over is a named barrier per (tile, quarter) over the two warps
     // (64 threads): the waiting warp is descheduled and polls nothing, so it
@@ -389,7 +389,7 @@ __global__ void __launch_bounds__(kThreadsFa, 1)
     // A named barrier has no timeout, so a warp that gives up (a bounded wait
     // ran out) still walks the rest of the hand-over sequence below the loop
     // and its partner is never left waiting.
-    const int n_paired = min(r0.hi - r0.lo, r1.hi - r1.lo);
+    const int n_paired = paired_blocks(r0, r1);
     const int my_turn = 1 + i * 4 + quarter;
     const int other_turn = 1 + (1 - i) * 4 + quarter;
     int turns_done = 0;  // hand-over steps this warp has completed

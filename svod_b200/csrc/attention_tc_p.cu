@@ -544,7 +544,7 @@ __global__ void __launch_bounds__(kThreadsFa, 1)
       if (lane == 0) mbar_arrive(&item_empty[slot]);
       if (!w.valid) break;
       if (!ok) {
-        const int pairs = min(w.r0.hi - w.r0.lo, w.r1.hi - w.r1.lo);
+        const int pairs = paired_blocks(w.r0, w.r1);
         // arrivals only: a partner still computing is released at each of its
         // turns, and this warp never waits on a barrier without a limit again
         for (int m = 0; m < pairs; ++m)
@@ -590,7 +590,7 @@ __global__ void __launch_bounds__(kThreadsFa, 1)
       // The hand-over of the MUFU unit between the two tiles (see the one-item
       // kernel): a named barrier per (tile, quarter); a warp that gave up still
       // walks the rest of the item's sequence.
-      const int n_paired = min(w.r0.hi - w.r0.lo, w.r1.hi - w.r1.lo);
+      const int n_paired = paired_blocks(w.r0, w.r1);
       int turns_done = 0;
       uint32_t sr[2][32];
       bool requested = false;

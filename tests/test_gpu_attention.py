@@ -742,3 +742,45 @@ def test_small_f16_weights_beside_appended_rows_stay_in_the_sum(T):
     assert "cluster:" in ops.chosen()
     rest = Tk * math.exp(-17.5)
     assert np.abs(got / (rest / (1.0 + rest)) - 1.0).max() < 2.0 ** -11 + 2.0 ** -16
+
+
+@pytest.mark.parametrize("H,Hkv,kw", [
+    (4, 2, dict(chunk=(1000, 0, 0))),          # one item at a time; a chunk border inside an item, 15 blocks on
+    (24, 24, dict(chunk=(900, 0, 0))),         # the persistent kernel, two tiles of a head
+    (12, 6, dict(chunk=(900, 1, 0))),          # the same, grouped heads paired: equal ranges
+    (2, 2, dict(causal=True, seg=True)),       # packed segments: the second tile begins where its segment does
+    (24, 24, dict(causal=True, seg=True)),
+])
+def test_tiles_of_an_item_whose_keys_begin_far_apart(H, Hkv, kw):
+    B, T, D, dt = 2, 2000, 64, O.BF16
+    rng = np.random.default_rng(H)
+    q, k, v = (normal(rng, (B, T, h, D), 1.0, dt) for h in (H, Hkv, Hkv))
+    seg = None
+    if kw.get("seg"):  # segments that begin inside items, short ones and padding rows of their own behind them
+        starts = np.array([0, 400, 896, 1025, 1030, 1500])
+        seg = starts[np.searchsorted(starts, np.arange(T), side="right") - 1]
+        seg[1900:] = np.arange(1900, T)
+        seg = np.tile(seg, (B, 1)).astype(np.int32)
+    j, i = np.arange(T)[None, :], np.arange(T)[:, None]
+    hide = np.zeros((B, T, T), bool)
+    a = ops.Attn(causal=bool(kw.get("causal")))
+    if a.causal:
+        hide |= j > i
+    if seg is not None:
+        hide |= j[None] < seg[:, :, None]
+        a.seg_start = torch.from_numpy(seg).cuda()
+    if "chunk" in kw:
+        size, left, right = kw["chunk"]
+        hide |= (j // size + left < i // size) | (j // size > i // size + right)
+        a.chunk = ops.Chunk(size, left, right)
+    got = ops.attention(dev(q, dt), dev(k, dt), dev(v, dt), a)
+    assert "kernel flash_attention" in ops.chosen()
+    ops.device_status()
+    Q, K, V = (dev(x, dt).double() for x in (q, k, v))
+    hd = torch.from_numpy(hide).cuda()
+    for b in range(B):
+        for h in range(H):
+            s = (Q[b, :, h] @ K[b, :, h // (H // Hkv)].T / math.sqrt(D)).masked_fill(hd[b], -math.inf)
+            want = s.softmax(-1) @ V[b, :, h // (H // Hkv)]
+            # 16-bit weights below 1 and a 16-bit result: two steps of 2^-8 of values up to 4
+            assert float((got[b, :, h].double() - want).abs().max()) < 3e-2
