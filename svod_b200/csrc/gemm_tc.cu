@@ -74,13 +74,13 @@ struct Params {
   int tma_epilogue;   // stage the output through shared memory and TMA-store it
   // Attention prologue in the store (the tile's column half is one 128-wide
   // head): RMSNorm over the head with `norm_q` for columns below norm_q_cols,
-  // `norm_k` below norm_cols, none above; then the rotation for columns below
+  // `norm_k` from norm_k_from to norm_cols, none elsewhere; then the rotation for columns below
   // rope_width; staged and TMA-stored like the plain epilogue.
   int head_epilogue;
   int head64_epilogue;  // the same for 64-wide heads: one head per 64-column sub-tile
   const void* norm_q;
   const void* norm_k;
-  int norm_q_cols, norm_cols;
+  int norm_q_cols, norm_k_from, norm_cols;
   float norm_eps;
   const int32_t* live;       // nullable: packed rows to compute; tiles past them are not walked
   const int32_t* block_pos;  // their blocks' positions
@@ -396,7 +396,8 @@ __global__ void __launch_bounds__(kThreads, 1)
           const int c0 = c_lo + sub * 64;
           const int h_col = n0 + c0;
           const bool turned = h_col < p.rope_width;
-          const float* nw = h_col < p.norm_q_cols ? head_w : (h_col < p.norm_cols ? head_w + 128 : nullptr);
+          const float* nw = h_col < p.norm_q_cols ? head_w
+                          : h_col >= p.norm_k_from && h_col < p.norm_cols ? head_w + 128 : nullptr;
           float a[32], b[32];
           acc32<T>(t_acc + (uint32_t)c0, bias, h_col, p.n, a);
           acc32<T>(t_acc + (uint32_t)(c0 + 32), bias, h_col + 32, p.n, b);
@@ -468,7 +469,8 @@ __global__ void __launch_bounds__(kThreads, 1)
         const int m0 = mt * BM;
         const int h_col = n0 + c_lo;  // first output column of this head
         const bool turned = head_turned;
-        const float* nw = h_col < p.norm_q_cols ? head_w : (h_col < p.norm_cols ? head_w + 128 : nullptr);
+        const float* nw = h_col < p.norm_q_cols ? head_w
+                        : h_col >= p.norm_k_from && h_col < p.norm_cols ? head_w + 128 : nullptr;
         const T* cos = (const T*)p.rope_cos;
         const T* sin = (const T*)p.rope_sin;
         const int64_t pos = rope_pos;
@@ -765,6 +767,7 @@ int launch_gemm_tc(const GemmArgs& a, cudaStream_t s, char* cfg, size_t cfg_len)
   p.norm_q = a.norm_q;
   p.norm_k = a.norm_k;
   p.norm_q_cols = a.norm_q != nullptr ? a.norm_q_heads * a.rope_head_dim : 0;
+  p.norm_k_from = a.norm_q_heads * a.rope_head_dim;  // (query heads without a weight of their own take none)
   p.norm_cols = a.norm_k != nullptr ? (a.norm_q_heads + a.norm_k_heads) * a.rope_head_dim : p.norm_q_cols;
   p.norm_eps = a.norm_eps;
   p.status = a.status;

@@ -71,10 +71,10 @@ struct Params2 {
   const void* residual;
   uint32_t* status;
   // head variant: per-head RMSNorm (weights norm_q below norm_q_cols, norm_k
-  // below norm_cols) and rotation (columns below rope_width) of 128-wide heads
+  // from norm_k_from to norm_cols) and rotation (columns below rope_width) of 128-wide heads
   const void* norm_q;
   const void* norm_k;
-  int norm_q_cols, norm_cols;
+  int norm_q_cols, norm_k_from, norm_cols;
   float norm_eps;
   int rope_width;
   int head_dim;      // 128 (norm and/or rotation), or 64 (rotation only)
@@ -480,7 +480,8 @@ __global__ void __launch_bounds__(32 * (2 + EW), 1)
         const int h_col = n0 + c_lo;
         const bool tile_tables = n0 < p.rope_width;
         const bool turned = h_col < p.rope_width;
-        const float* nw = h_col < p.norm_q_cols ? head_w : (h_col < p.norm_cols ? head_w + 128 : nullptr);
+        const float* nw = h_col < p.norm_q_cols ? head_w
+                        : h_col >= p.norm_k_from && h_col < p.norm_cols ? head_w + 128 : nullptr;
         const uint32_t t_head = t_acc + (uint32_t)c_lo;
         float inv = 1.f;
         if (nw != nullptr) {
@@ -689,6 +690,7 @@ int run2(const GemmArgs& a, int sms, cudaStream_t s, char* cfg, size_t cfg_len) 
   if (HEADS) {
     p.norm_q = a.norm_q, p.norm_k = a.norm_k;
     p.norm_q_cols = a.norm_q != nullptr ? a.norm_q_heads * 128 : 0;
+    p.norm_k_from = a.norm_q_heads * 128;
     p.norm_cols = a.norm_k != nullptr ? (a.norm_q_heads + a.norm_k_heads) * 128 : p.norm_q_cols;
     p.norm_eps = a.norm_eps;
     p.head_dim = a.rope_cos != nullptr && a.rope_head_dim == 64 ? 64 : 128;

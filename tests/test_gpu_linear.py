@@ -7,6 +7,7 @@ import pytest
 import torch
 
 from oracle import svod_oracle as O
+from svod_b200 import _lib as L
 from svod_b200 import ops
 from tests.test_oracle_pins import EPILOGUES, gemm_recipe
 from tests.util import dev, host, max_abs, mean_rel, rel_close
@@ -450,3 +451,38 @@ def test_few_tile_calls_match_f64(m, n, k, gated, tile):
     # one rounding to bf16 (2^-9 of the value at most), f32 sums below that
     assert ((got.double() - want).abs() <= 2.0 ** -8 * want.abs() + 1e-3).all()
     assert torch.equal(got, ops.linear(x, w, opts))  # partials are summed in a fixed order
+
+
+@pytest.mark.parametrize("qn,kn", [(False, True), (True, False)])
+@pytest.mark.parametrize("T,hd,rope,form", [
+    (100, 128, True, "cluster:"), (100, 64, True, "cluster:"),      # the few-tile kernel
+    (1500, 128, True, "bn:256"), (1500, 64, False, "bn:"),          # one CTA a tile
+    (9088, 128, True, "cta_pair:1"), (9000, 128, False, "cta_pair:1"),
+])
+def test_heads_without_a_norm_weight_are_not_normalised(T, hd, rope, form, qn, kn):
+    """Only q or only k has norm weights: the other's heads are turned as they are, whichever
+    kernel the size takes."""
+    H, Hkv, k, dt = 8, 4, 256, torch.bfloat16
+    g = torch.Generator(device="cuda").manual_seed(T + hd)
+    r = lambda *s: torch.randn(*s, generator=g, device="cuda")
+    x, w = r(1, T, k).to(dt), (r((H + 2 * Hkv) * hd, k) / 8).to(dt)  # heads of a norm far from 1
+    nw = (1 + 0.2 * r(hd)).to(dt)
+    c, s = ops.rope_table(1e4, T, hd, dt)
+    tabs = (c.view(1, T, 1, hd // 2), s.view(1, T, 1, hd // 2)) if rope else None
+    opts = ops.Linear(qkv=ops.Qkv(H, Hkv, hd, nw if qn else None, nw if kn else None, 1e-6, tabs))
+    got, lib = ops.linear(x, w, opts), L.load()
+    if form == "cta_pair:1":
+        lib.svodb_config_set(lib.svodb_last_config_key(), 512)
+        got = ops.linear(x, w, opts)
+        lib.svodb_config_clear()
+    assert form in ops.chosen(), ops.chosen()
+    z = (x.double() @ w.double().T).view(T, H + 2 * Hkv, hd)
+    norm = lambda v: v * torch.rsqrt((v * v).mean(-1, keepdim=True) + 1e-6) * nw.double()
+    parts = [norm(z[:, :H]) if qn else z[:, :H], norm(z[:, H:H + Hkv]) if kn else z[:, H:H + Hkv], z[:, H + Hkv:]]
+    if rope:
+        cd, sd = c.double()[:, None], s.double()[:, None]
+        turn = lambda v: torch.cat([v[..., :hd // 2] * cd - v[..., hd // 2:] * sd, v[..., :hd // 2] * sd + v[..., hd // 2:] * cd], -1)
+        parts[:2] = [turn(v) for v in parts[:2]]
+    want = torch.cat(parts, 1).view(1, T, -1)
+    # one rounding to bf16 of an f32 result: 2^-9 of the value, cancellation in the turn below 1e-3 of the head
+    assert ((got.double() - want).abs() <= 2.0 ** -8 * want.abs() + 4e-3).all()
