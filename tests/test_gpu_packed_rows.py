@@ -50,12 +50,13 @@ CASES = [
 
 
 def _close(got, want, kind):
-    # the same roundings of the same values; only the order of a row's key blocks' rescaling may differ
-    tol = {"xlmr": 2e-3, "qwen3": 1.5e-2, "modernbert": 1.2e-2}[kind]
+    # the same values bit for bit up to the pooling, whose f32 mean of up to 1024 tokens may be summed in
+    # another order: 1024 * 2^-24 (a key block missing from one row of a batch is 1e-2 of that row)
+    tol = 1024 * 2.0 ** -24
     got, want = got.double().cpu(), want.double().cpu()
     assert torch.isfinite(got).all()
     assert (got - want).norm() <= tol * want.norm()
-    assert ((got - want).norm(dim=1) <= 2 * tol * want.norm(dim=1).clamp_min(1e-30)).all()
+    assert ((got - want).norm(dim=1) <= tol * want.norm(dim=1).clamp_min(1e-30)).all()
 
 
 @pytest.mark.parametrize("kind", STACKS)
