@@ -316,6 +316,13 @@ def step_flops(kind: str, batch: int, seq: int):
     return gemm, attn
 
 
+def rows_flops(kind: str, lens):
+    """`step_flops` of rows of these lengths: the stacks compute a padded batch's rows
+    without their trailing padding, so that is the work of a step."""
+    per_row = [step_flops(kind, 1, int(n)) for n in lens]
+    return sum(g for g, _ in per_row), sum(a for _, a in per_row)
+
+
 def time_kernel(fn, stream, reps: int):
     import torch
     for _ in range(3):
@@ -553,10 +560,10 @@ def gpu_arm(args):
     ids_host, aux_host, lens = synthetic_batch(kind, batch, seq, vocab, 1234 + rank, ragged=False)
     run, m = measure_stack(kind, model, aux_kind, batch, seq, world, rank, device, args, ids_host, aux_host, True)
     ms_step, e2e_ms, clocks = m["ms_per_step"], m["e2e_ms"], m["clocks"]
-    tokens_step = batch * seq * world
+    real_tokens = int(lens.sum())
+    tokens_step = real_tokens * world  # padding is not computed and not counted
     value = tokens_step / (ms_step * 1e-3)
     e2e_value = tokens_step / (e2e_ms * 1e-3)
-    real_tokens = int(lens.sum())
     launches_per_step = run.launches_per_step
     run_collective = run.collective
     h2d, d2h = run.h2d_bytes(), run.out_host.numel() * 4
@@ -582,12 +589,12 @@ def gpu_arm(args):
         srun, sm = measure_stack(kind, model, aux_kind, per, seq, world, rank, device, args, g_ids[my_rows],
                                  g_aux[my_rows], False)
         s_ms = sm["ms_per_step"]
-        strong = {"tokens_per_s": batch * seq / (s_ms * 1e-3), "ms_per_step": s_ms, "rows_per_gpu": per,
-                  "global_batch": batch, "e2e_tokens_per_s": batch * seq / (sm["e2e_ms"] * 1e-3),
-                  "n1_ms_per_step": ms_step, "speedup_vs_n1": ms_step / s_ms, "efficiency_vs_n1": ms_step / s_ms / world,
-                  "note": ("one batch of ragged rows dealt longest-first round-robin (shard_rows); n1 = this run's "
-                           "own full-batch step on one GPU (the weak pass: the same work, since a Qwen3 row's length "
-                           "only moves its pooled position); all-gather inside the captured graph")}
+        g_tokens = int(g_lens.sum())
+        strong = {"tokens_per_s": g_tokens / (s_ms * 1e-3), "ms_per_step": s_ms, "rows_per_gpu": per,
+                  "global_batch": batch, "e2e_tokens_per_s": g_tokens / (sm["e2e_ms"] * 1e-3),
+                  "note": ("one batch of ragged rows dealt longest-first round-robin (shard_rows), real tokens; the weak "
+                           "pass is no one-GPU reference for it (its rows are full length, and padding is not "
+                           "computed); all-gather inside the captured graph")}
         if rank == 0:
             undone = E.unshard_rows(srun.gathered, shards)   # back to the batch's own row order
             strong["matches_one_gpu_rows"] = bool(torch.equal(undone, full_rows))
@@ -616,7 +623,7 @@ def gpu_arm(args):
         e1.record(nstream)
         nstream.synchronize()
         nms = e0.elapsed_time(e1) / args.steps
-        native = {"value": batch * seq / (nms * 1e-3), "unit": UNIT, "ms_per_step": nms,
+        native = {"value": real_tokens / (nms * 1e-3), "unit": UNIT, "ms_per_step": nms,
                   "api": "svodb_plan_run: host ids/lengths -> captured graph -> host pooled rows",
                   "matches_python_stack": bool((out_np == ref_rows).all())}
         runner.close()
@@ -624,7 +631,7 @@ def gpu_arm(args):
 
     line = None
     if rank == 0:
-        gemm_fl, attn_fl = step_flops(kind, batch, seq)
+        gemm_fl, attn_fl = rows_flops(kind, lens)
         line = {
             "metric": METRIC, "value": value, "unit": UNIT, "n_gpus": world, "steps": args.steps,
             "warmup": max(3, args.warmup), "ms_per_step": ms_step, "higher_is_better": True, "scaling": "weak",
@@ -696,9 +703,9 @@ def gpu_arm(args):
 
 
 def other_workloads(args, device, peaks):
-    """The two other encoder configurations on one GPU, a few steps each: padded
-    and real tokens/s (real = the tokens under the padding mask), step TFLOP/s and
-    the per-launch timing of their attention and largest GEMM."""
+    """The two other encoder configurations on one GPU, a few steps each: tokens/s and
+    step TFLOP/s of the real tokens (those under the padding mask; the padding behind
+    them is not computed) and the per-launch timing of their attention and largest GEMM."""
     import torch
     from svod_b200 import ops
     out = {}
@@ -708,11 +715,11 @@ def other_workloads(args, device, peaks):
         ids_host, aux_host, lens = synthetic_batch(kind, batch, seq, model.cfg.vocab_size, 1234, ragged=False)
         run, m = measure_stack(kind, model, aux_kind, batch, seq, 1, 0, device, args, ids_host, aux_host, True)
         ms = m["ms_per_step"]
-        gemm_fl, attn_fl = step_flops(kind, batch, seq)
+        gemm_fl, attn_fl = rows_flops(kind, lens)
+        tokens = int(lens.sum())
         rec = {"batch": batch, "seq_len": seq, "dtype": "f16" if kind == "xlmr" else "bf16", "ms_per_step": ms,
-               "tokens_per_s": batch * seq / (ms * 1e-3), "real_tokens_per_s": int(lens.sum()) / (ms * 1e-3),
-               "real_tokens_per_step": int(lens.sum()),
-               "e2e_tokens_per_s": batch * seq / (m["e2e_ms"] * 1e-3), "step_tflops_padded": (gemm_fl + attn_fl) / ms / 1e9,
+               "tokens_per_s": tokens / (ms * 1e-3), "real_tokens_per_step": tokens,
+               "e2e_tokens_per_s": tokens / (m["e2e_ms"] * 1e-3), "step_tflops": (gemm_fl + attn_fl) / ms / 1e9,
                "gpu_launches_per_step": run.launches_per_step, "clocks": m["clocks"], "output_finite": m["finite"]}
         del run, model
         torch.cuda.empty_cache()

@@ -258,42 +258,42 @@ __global__ void __launch_bounds__(256)
   }
   const int64_t step = (int64_t)warps * csz;
   for (int64_t t0 = first + share * warps + warp; t0 < last; t0 += 32 * step) {
-   // 32 of the warp's tokens at a time: which of them are real, then those one by one
-   const int64_t tl = t0 + lane * step;
-   bool real = tl < last;
-   if (mode == 1 && real)
-     real = (aux_i32 ? ((const int32_t*)aux)[bi * l_len + tl] : (int)((const uint8_t*)aux)[bi * l_len + tl]) != 0;
-   uint32_t todo = __ballot_sync(0xffffffffu, real);
-   cnt += (float)__popc(todo);
-   uint4 u[SPANS];
-   auto fetch = [&]() {
-     const T* src = h + (t0 + (__ffs((int)todo) - 1) * step) * D + lane * 8;
+    // 32 of the warp's tokens at a time: which of them are real, then those one by one
+    const int64_t tl = t0 + lane * step;
+    bool real = tl < last;
+    if (mode == 1 && real)
+      real = (aux_i32 ? ((const int32_t*)aux)[bi * l_len + tl] : (int)((const uint8_t*)aux)[bi * l_len + tl]) != 0;
+    uint32_t todo = __ballot_sync(0xffffffffu, real);
+    cnt += (float)__popc(todo);
+    uint4 u[SPANS];
+    auto fetch = [&]() {
+      const T* src = h + (t0 + (__ffs((int)todo) - 1) * step) * D + lane * 8;
 #pragma unroll
-     for (int s = 0; s < SPANS; ++s) u[s] = ldg128(src + s * 256);
-   };
-   if (todo != 0u) fetch();
-   while (todo != 0u) {
-    float v[SPANS][8];
-#pragma unroll
-    for (int s = 0; s < SPANS; ++s) rows_parts::unpack8<T>(u[s], v[s]);
-    todo &= todo - 1;
+      for (int s = 0; s < SPANS; ++s) u[s] = ldg128(src + s * 256);
+    };
     if (todo != 0u) fetch();
-    if (w != nullptr) {
-      const float inv = rows_parts::centre_and_scale<SPANS>(v, eps, layer);
+    while (todo != 0u) {
+      float v[SPANS][8];
 #pragma unroll
-      for (int s = 0; s < SPANS; ++s) {
-        const int off = s * 256 + lane * 8;
-        float y[8];
-        rows_parts::affine8<T>(v[s], inv, ldg128(w + off), b != nullptr ? ldg128(b + off) : make_uint4(0, 0, 0, 0),
-                               b != nullptr, y);
-        rows_parts::unpack8<T>(rows_parts::pack8<T>(y), v[s]);  // the 16-bit value the norm would store
+      for (int s = 0; s < SPANS; ++s) rows_parts::unpack8<T>(u[s], v[s]);
+      todo &= todo - 1;
+      if (todo != 0u) fetch();
+      if (w != nullptr) {
+        const float inv = rows_parts::centre_and_scale<SPANS>(v, eps, layer);
+#pragma unroll
+        for (int s = 0; s < SPANS; ++s) {
+          const int off = s * 256 + lane * 8;
+          float y[8];
+          rows_parts::affine8<T>(v[s], inv, ldg128(w + off), b != nullptr ? ldg128(b + off) : make_uint4(0, 0, 0, 0),
+                                 b != nullptr, y);
+          rows_parts::unpack8<T>(rows_parts::pack8<T>(y), v[s]);  // the 16-bit value the norm would store
+        }
       }
+#pragma unroll
+      for (int s = 0; s < SPANS; ++s)
+#pragma unroll
+        for (int i = 0; i < 8; ++i) acc[s][i] += v[s][i];
     }
-#pragma unroll
-    for (int s = 0; s < SPANS; ++s)
-#pragma unroll
-      for (int i = 0; i < 8; ++i) acc[s][i] += v[s][i];
-   }
   }
   if (warps > 1) {
 #pragma unroll
