@@ -681,7 +681,7 @@ int run_dec(const AttnArgs& a, cudaStream_t s, char* cfg, size_t cfg_len) {
   const int64_t pairs = a.batch * a.kv_heads;
   const int csize = dec_cluster(pairs, dec_blocks(a), C::kPerSm);
   if (launch_pdl(attention_decode_kernel<T, D, NQ>, dim3((unsigned)(pairs * csize)), dim3(kThreadsDec), C::kSmem, s,
-                 (unsigned)csize, tk, tv, tka, tva, p) != cudaSuccess)
+                 (unsigned)csize, a.batch * a.t, tk, tv, tka, tva, p) != cudaSuccess)
     return -1;
   if (cfg != nullptr)
     snprintf(cfg, cfg_len, "{rows:%d,bkv:%d,d:%d,stages:%d,splits:1,cluster:%d}", NQ, kKeys, a.d, C::kSlots, csize);

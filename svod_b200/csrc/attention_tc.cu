@@ -655,7 +655,8 @@ int run(const AttnArgs& a, cudaStream_t s, char* cfg, size_t cfg_len) {
   p.d_real = a.d;
   p.status = a.status;
   dim3 grid((unsigned)p.n_qt, (unsigned)a.heads, (unsigned)a.batch);
-  if (launch_pdl(attention_tc_kernel<T, D>, grid, dim3(kThreadsFa), C::kSmemBytes, s, 1, tq, tk, tv, p) != cudaSuccess)
+  if (launch_pdl(attention_tc_kernel<T, D>, grid, dim3(kThreadsFa), C::kSmemBytes, s, 1, a.batch * a.t, tq, tk, tv, p) !=
+      cudaSuccess)
     return -1;
   if (cfg != nullptr)
     snprintf(cfg, cfg_len, "{bq:%d,bkv:%d,d:%d,stages:%d,splits:1}", 2 * kBQ, kBKV, a.d, C::kStages);

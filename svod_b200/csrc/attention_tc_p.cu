@@ -965,8 +965,8 @@ int run_p(const AttnArgs& a, cudaStream_t s, char* cfg, size_t cfg_len) {
     const int64_t want = (6 * (int64_t)sms + per_kv - 1) / per_kv;
     tail_groups = (int)(want < groups ? want : groups);
   }
-  if (launch_pdl(attention_tc_p_kernel<T, D, EXTRAS>, dim3((unsigned)grid), dim3(kThreadsFa), smem_bytes_p<D>(), s, 1, tq, tk,
-                 tv, to, p, (int)items, tail_groups, head) != cudaSuccess)
+  if (launch_pdl(attention_tc_p_kernel<T, D, EXTRAS>, dim3((unsigned)grid), dim3(kThreadsFa), smem_bytes_p<D>(), s, 1,
+                 a.batch * a.t, tq, tk, tv, to, p, (int)items, tail_groups, head) != cudaSuccess)
     return -1;
   if (cfg != nullptr)
     snprintf(cfg, cfg_len, p.pair_heads ? "{bq:%d,bkv:%d,d:%d,stages:%d,splits:%d,persistent:%d,head_pairs:1}"

@@ -445,8 +445,8 @@ int run_s(const GemmArgs& a, int splits, cudaStream_t s, char* cfg, size_t cfg_l
     attr_seen[dev & 63] = true;
   }
   const int grid = p.tiles_m * tiles_n * splits;
-  if (launch_pdl(gemm_small_kernel<T, BN>, dim3((unsigned)grid), dim3(kThreads), smem, s, (unsigned)splits, ta, tw, p) !=
-      cudaSuccess)
+  if (launch_pdl(gemm_small_kernel<T, BN>, dim3((unsigned)grid), dim3(kThreads), smem, s, (unsigned)splits, a.m, ta, tw,
+                 p) != cudaSuccess)
     return -1;
   if (cfg != nullptr)
     snprintf(cfg, cfg_len, "{bm:%d,bn:%d,bk:%d,stages:%d,gated:%d,grid:%d,cluster:%d}", BM, BN, BK, p.stages, a.gated, grid,

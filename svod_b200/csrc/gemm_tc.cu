@@ -694,8 +694,8 @@ int run(const GemmArgs& a, const Params& p0, int sms, cudaStream_t s, char* cfg,
   }
   const int tiles = p.tiles_m * p.tiles_n;
   const int grid = tiles < sms ? tiles : sms;
-  if (launch_pdl(gemm_tc_kernel<T, BN>, dim3((unsigned)grid), dim3(kThreads), C::kSmemBytes, s, 1, ta, tw, tc, tr, p) !=
-      cudaSuccess)
+  if (launch_pdl(gemm_tc_kernel<T, BN>, dim3((unsigned)grid), dim3(kThreads), C::kSmemBytes, s, 1, a.m, ta, tw, tc, tr,
+                 p) != cudaSuccess)
     return -1;
   if (cfg != nullptr)
     snprintf(cfg, cfg_len, "{bm:%d,bn:%d,bk:%d,stages:%d,gated:%d,grid:%d}", BM, BN, BK, C::kStages, a.gated, grid);

@@ -718,8 +718,8 @@ int run2(const GemmArgs& a, int sms, cudaStream_t s, char* cfg, size_t cfg_len) 
   }
   const int tiles = p.tiles_m * p.tiles_n;
   const int pairs = tiles < sms / 2 ? tiles : sms / 2;
-  if (launch_pdl(gemm_tc2_kernel<T, HEADS, EW>, dim3((unsigned)(2 * pairs)), dim3(C::kThreads), C::kSmemBytes, s, 2, ta, tw,
-                 tc, tr, tcos, tsin, p) != cudaSuccess)
+  if (launch_pdl(gemm_tc2_kernel<T, HEADS, EW>, dim3((unsigned)(2 * pairs)), dim3(C::kThreads), C::kSmemBytes, s, 2, a.m, ta,
+                 tw, tc, tr, tcos, tsin, p) != cudaSuccess)
     return -1;
   if (cfg != nullptr)
     snprintf(cfg, cfg_len, "{bm:%d,bn:%d,bk:%d,stages:%d,gated:%d,grid:%d,cta_pair:1,epi_warps:%d}", 2 * BM, BN, BK,

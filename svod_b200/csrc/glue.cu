@@ -475,7 +475,7 @@ void launch_embed(const EmbedArgs& a, cudaStream_t s) {
   dim3 grid((unsigned)(((a.layout != nullptr ? lay.len : a.t) + kTok - 1) / kTok), (unsigned)a.batch);
   const int vec16 = aligned16(a.table) && aligned16(a.pos_table) && aligned16(a.type_row) && aligned16(a.out) ? 1 : 0;
 #define SVODB_EMBED(T, I)                                                                                         \
-  launch_pdl(embed_kernel<T, I>, grid, dim3(256), 0, s, 1, (const I*)a.ids, (const T*)a.table,         \
+  launch_pdl(embed_kernel<T, I>, grid, dim3(256), 0, s, 1, a.batch * a.t, (const I*)a.ids, (const T*)a.table, \
              (const T*)a.pos_table, (const T*)a.type_row, a.pad_id, (T*)a.out, a.t, a.d, a.vocab, a.max_pos, vec16, lay.live, \
              lay.block_seq, lay.block_pos)
   if (a.dtype == SVODB_BF16) {
@@ -496,9 +496,9 @@ bool embed_norm_dispatch(const EmbedArgs& a, const EmbedNormArgs& n, cudaStream_
   dim3 grid((unsigned)(((a.layout != nullptr ? lay.len : a.t) + kTok - 1) / kTok), (unsigned)a.batch);
 #define SVODB_EN(SP)                                                                                                \
   case SP:                                                                                                          \
-    launch_pdl(embed_norm_kernel<T, I, SP>, grid, dim3(kTok * 32), 0, s, 1, (const I*)a.ids, (const T*)a.table,      \
+    launch_pdl(embed_norm_kernel<T, I, SP>, grid, dim3(kTok * 32), 0, s, 1, a.batch * a.t, (const I*)a.ids, (const T*)a.table, \
                (const T*)a.pos_table, (const T*)a.type_row, a.pad_id, (const T*)n.w, (const T*)n.b, n.eps, n.layer, \
-               (T*)a.out, a.t, a.vocab, a.max_pos, lay.live, lay.block_seq, lay.block_pos);                                                                \
+               (T*)a.out, a.t, a.vocab, a.max_pos, lay.live, lay.block_seq, lay.block_pos); \
     return true
   switch (a.d / 256) {
     SVODB_EN(1); SVODB_EN(2); SVODB_EN(3); SVODB_EN(4); SVODB_EN(5); SVODB_EN(6); SVODB_EN(7); SVODB_EN(8);
@@ -521,9 +521,9 @@ bool norm_pool_dispatch(const PoolArgs& a, const EmbedNormArgs& n, cudaStream_t 
   const PeerPush pp = a.push != nullptr ? *a.push : PeerPush{};
 #define SVODB_NP(SP)                                                                                               \
   case SP:                                                                                                         \
-    launch_pdl(norm_pool_kernel<T, SP>, dim3((unsigned)(out_rows * blocks)), dim3(warps * 32), 0, s, blocks, (const T*)a.hidden,    \
+    launch_pdl(norm_pool_kernel<T, SP>, dim3((unsigned)(out_rows * blocks)), dim3(warps * 32), 0, s, blocks, a.batch * a.l, (const T*)a.hidden, \
                (const T*)n.w, (const T*)n.b, n.eps, n.layer, a.aux, a.aux_i32, a.mode, a.slots, a.normalize, a.out, \
-               a.out_row_stride, a.l, pp, a.row_start, a.row_keys);                                                                         \
+               a.out_row_stride, a.l, pp, a.row_start, a.row_keys); \
     return true
   switch (spans) {
     SVODB_NP(1); SVODB_NP(2); SVODB_NP(3); SVODB_NP(4); SVODB_NP(5); SVODB_NP(6); SVODB_NP(7); SVODB_NP(8);

@@ -157,7 +157,7 @@ void run(const HeadsArgs& a, cudaStream_t s) {
   const int64_t tokens = a.batch * a.t;
   const int64_t threads = tokens * (a.heads + 2 * a.kv_heads) * LPH;
   const unsigned blocks = (unsigned)((threads + 255) / 256);
-  launch_pdl(heads_kernel<T, LPH>, dim3(blocks), dim3(256), 0, s, 1, (const T*)a.qkv, (const T*)a.q_w, (const T*)a.k_w,
+  launch_pdl(heads_kernel<T, LPH>, dim3(blocks), dim3(256), 0, s, 1, tokens, (const T*)a.qkv, (const T*)a.q_w, (const T*)a.k_w,
              (const T*)a.cos, (const T*)a.sin, (T*)a.q, (T*)a.k, (T*)a.v, tokens, a.t, a.heads, a.kv_heads, a.eps,
              a.per_batch_tables, a.in_place);
 }

@@ -145,7 +145,7 @@ RowLayout row_layout_of(int64_t batch, int64_t len, const int32_t* table) {
 }
 
 void launch_row_layout(const RowLayoutArgs& a, cudaStream_t s) {
-  launch_pdl(row_layout_kernel, dim3((unsigned)a.batch), dim3(kLayoutThreads), 0, s, 1, a, padded_len(a.len));
+  launch_pdl(row_layout_kernel, dim3((unsigned)a.batch), dim3(kLayoutThreads), 0, s, 1, a.batch * a.len, a, padded_len(a.len));
 }
 
 }  // namespace svodb

@@ -150,7 +150,7 @@ void run_rows(const NormArgs& a, cudaStream_t s) {
   const int per_sm = rows_blocks(SPANS, a.residual != nullptr);
   const unsigned blocks = (unsigned)(want < (int64_t)sms * per_sm ? want : (int64_t)sms * per_sm);
   auto* kernel = a.residual != nullptr ? norm_rows_kernel<T, SPANS, true> : norm_rows_kernel<T, SPANS, false>;
-  launch_pdl(kernel, dim3(blocks), dim3(kWarpsPerBlock * 32), 0, s, 1, (const T*)a.x, (const T*)a.residual, (const T*)a.w,
+  launch_pdl(kernel, dim3(blocks), dim3(kWarpsPerBlock * 32), 0, s, 1, a.rows, (const T*)a.x, (const T*)a.residual, (const T*)a.w,
              (const T*)a.b, (T*)a.out, (T*)a.sum, a.rows, a.eps, a.layer, a.live);
 }
 
