@@ -3,9 +3,10 @@
 //
 // What bounds it: the cache. B8 x Tk 32768 x 8 KV heads x 128 is 1.03 GB of keys and
 // values for 2 query rows each. The 256-row tile kernel (attention_tc_p.cu) spends its
-// time on the exponentials of 254 rows nobody asked for (415 us); here it takes 151 us,
-// 6.8 TB/s. Appended cache rows used to go to the exact kernel, on scalar loads (B24,
-// 150..2048 keys + 5, 8 KV heads x 64: 1120 us; 18 us here).
+// time on the exponentials of 254 rows nobody asked for (416 us with lengths from 30000);
+// here it takes 160 us, 6.46 TB/s of the keys it reads (a plain copy: 6.54). Appended cache
+// rows used to go to the exact kernel, on scalar loads (B24, 150..2048 keys + 5, 8 KV heads
+// x 64: 1114 us; 19 us here).
 //
 // How it is laid out for that: keys are the M dimension of both contractions, so
 // a 128-key block costs two small MMAs whatever the number of query rows:
@@ -534,7 +535,9 @@ __global__ void __launch_bounds__(kThreadsDec, (DecCfg<D, NQ>::kPerSm))
           tmem_ld_cols(o_tmem + NQ + q0, lo);
 #pragma unroll
           for (int c = 0; c < 16; ++c)
-            if (q0 + c < p.rows) op[(q0 + c) * D + tid] = fmaf(__uint_as_float(lo[c]), 1.f / kRestUp<T>, __uint_as_float(sr[c])) * (1.f / kValueUp<T>);
+            if (q0 + c < p.rows)
+              op[(q0 + c) * D + tid] =
+                  fmaf(__uint_as_float(lo[c]), 1.f / kRestUp<T>, __uint_as_float(sr[c])) * (1.f / kValueUp<T>);
         }
         if (NQ == 16) break;
       }

@@ -2,8 +2,8 @@
 // exact path (attention_generic.cu keeps every other type, head dim, bias, key splits and
 // appended rows). f32 products, sums and exponentials throughout, as there.
 //
-// What bounds it: the FMA pipe (B2 x H8 x 512 x 512 x 64 is 0.5 G multiply-adds in each
-// product, about 14 us at the chip's rate). The generic kernel read two shared-memory words
+// What bounds it: the FMA pipe (B2 x H8 x 512 x 512 x 64 is 0.27 G multiply-adds in each
+// product, 14 us for both at the chip's 37 T a second, 13 for the keys of the case below). The generic kernel read two shared-memory words
 // per multiply-add (232 us with key lengths 256..512, 34 here; B4 x H8 x 1024 x 1024 x 128
 // 2278 -> 417 us, 31 TFLOP/s; B2 x 20 queries x 1000 keys 378 -> 19 us). Here a thread
 // owns 4 query rows x 4 keys of a 64 x 64 score tile and 4 rows x D/16 columns of the output,

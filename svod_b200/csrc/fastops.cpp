@@ -291,7 +291,8 @@ PyObject* attention_packed(PyObject*, PyObject* const* args, Py_ssize_t n) {
   desc_of(out, y, x.dtype);
   if (want) lse = lse_for(xt, x.shape[0], heads, x.shape[1], o, keep);
   void* st = stream();
-  if (unlocked([&] { return p_attention_packed(&x, (int32_t)heads, (int32_t)kv, &o, &y, st); }) != SVODB_OK) return none();
+  if (unlocked([&] { return p_attention_packed(&x, (int32_t)heads, (int32_t)kv, &o, &y, st); }) != SVODB_OK)
+    return none();
   return with_lse(std::move(out), std::move(lse), want);
   END_HANDLE_TH_ERRORS
 }
